@@ -294,7 +294,10 @@ PDFP_API int pdfp_get_tuning_seg(const pdfp_handle* h, int32_t* out);
  * from a captured graph; 1, one cooperative launch of the per-block row passes
  * (PDFP_MEDIUM=1); 2, one cooperative launch of the vec engine's warp items
  * (PDFP_VEC_WINDOW=1, both FP32 sides on the vec engine without long-row
- * pieces); 3, whole windows of each small member in one block's launch. */
+ * pieces); 3, whole windows of each small member in one block's launch; 4, steps
+ * 2 .. freq in one cooperative launch with the whole handle in the SMs' shared
+ * memory (where it fits there and no switch names another form or engine;
+ * PDFP_RESIDENT=0 switches it off). */
 PDFP_API int pdfp_get_window_form(const pdfp_handle* h, int32_t* out);
 /* Every measurement the autotuner took: up to `cap` rows, ms[i] the mean
  * launch time, cfg[7i..7i+6] = {side (0: A', 1: A), stage bytes, gatherer

@@ -256,6 +256,69 @@ bool DeviceMatrix::make_seg(DeviceArena& ar, int nseg, int long_min, const Stage
     return true;
 }
 
+bool DeviceMatrix::make_resident(DeviceArena& ar, int n_blocks, int esize, int ncv, int nrv,
+                                 int par_bytes, uint32_t max_smem, Resident& r) const {
+    r = Resident();
+    // entries and vectors alone, spread evenly: no need to lay out what cannot fit
+    const double least = 2.0 * L.NNZ * (4 + esize) + 1.0 * L.NNZ * esize +
+                         static_cast<double>(esize * ncv + 4) * L.N + static_cast<double>(esize * nrv + 4) * L.M;
+    if (n_blocks <= 0 || least > static_cast<double>(n_blocks) * max_smem) return false;
+    HostResident ht, ha;
+    deal_resident(L.At, L.col_off, n_blocks, ht);
+    deal_resident(L.A, L.row_off, n_blocks, ha);
+    for (int shared = 0; shared < 2 && (shared == 0 || r.smem > max_smem); ++shared) {
+        r.smem = 0;
+        r.shared = shared != 0;
+        for (int b = 0; b < n_blocks; ++b)
+            r.smem = std::max(r.smem, res_smem(ht.blocks[b], ha.blocks[b], esize, ncv, nrv, par_bytes, r.shared).total);
+    }
+    if (r.smem > max_smem) return false;
+    ::pdfp::fill_resident(L.At, ht);
+    ::pdfp::fill_resident(L.A, ha);
+    const std::vector<void*> d = ar.upload_group(
+        {part(ht.blocks), part(ht.slices), part(ht.longs), part(ht.lane_row), part(ht.idx), part(ht.src),
+         part(ha.blocks), part(ha.slices), part(ha.longs), part(ha.lane_row), part(ha.idx), part(ha.src)});
+    auto side = [&](int k) {
+        ResDev s;
+        s.blocks = static_cast<const ResBlock*>(d[k]);
+        s.slices = static_cast<const ResSlice*>(d[k + 1]);
+        s.longs = static_cast<const ResLong*>(d[k + 2]);
+        s.lane_row = static_cast<const int32_t*>(d[k + 3]);
+        s.idx = static_cast<const int32_t*>(d[k + 4]);
+        return s;
+    };
+    r.t = side(0);
+    r.a = side(6);
+    r.src_t = static_cast<const int32_t*>(d[5]);
+    r.src_a = static_cast<const int32_t*>(d[11]);
+    r.n_t = static_cast<int64_t>(ht.src.size());
+    r.n_a = static_cast<int64_t>(ha.src.size());
+    r.n_blocks = n_blocks;
+    return true;
+}
+
+template <typename T>
+__global__ void gather_values_kernel(const int32_t* __restrict__ src, const T* __restrict__ val,
+                                     T* __restrict__ out, int64_t n) {
+    for (int64_t i = blockIdx.x * int64_t(256) + threadIdx.x; i < n; i += int64_t(gridDim.x) * 256)
+        out[i] = src[i] >= 0 ? val[src[i]] : T(0);
+}
+
+template <typename T>
+static const void* resident_values(DeviceArena& ar, const int32_t* src, const T* val, int64_t n,
+                                   cudaStream_t s) {
+    T* out = ar.alloc<T>(n);
+    const int blocks = static_cast<int>(std::min<int64_t>((n + 255) / 256, 4096));
+    if (n > 0) gather_values_kernel<T><<<blocks, 256, 0, s>>>(src, val, out, n);
+    PDFP_CK(cudaGetLastError());
+    return out;
+}
+
+void DeviceMatrix::fill_resident(DeviceArena& ar, Resident& r, bool f32, cudaStream_t s) const {
+    r.t.val = f32 ? resident_values(ar, r.src_t, v32_t, r.n_t, s) : resident_values(ar, r.src_t, v64_t, r.n_t, s);
+    r.a.val = f32 ? resident_values(ar, r.src_a, v32_a, r.n_a, s) : resident_values(ar, r.src_a, v64_a, r.n_a, s);
+}
+
 VecDev DeviceMatrix::make_vec(DeviceArena& ar, bool transpose, int lane_nnz, int64_t min_items) const {
     const HostCsr& csr = transpose ? L.At : L.A;
     const std::vector<int32_t>& off = transpose ? L.col_off : L.row_off;

@@ -176,6 +176,21 @@ class DeviceMatrix {
     // (build_vec_items), with zeroed piece slots and counters; items of four times the
     // default rows when min_items > 0 and that still gives at least min_items items.
     VecDev make_vec(DeviceArena& ar, bool transpose, int lane_nnz, int64_t min_items) const;
+    // The resident window's layout of both sides (deal_resident) for n_blocks blocks,
+    // without its values; false when a block's share of either side would need more than
+    // max_smem bytes of shared memory.
+    struct Resident {
+        ResDev t, a;
+        const int32_t *src_t = nullptr, *src_a = nullptr;  // CSR position of each entry (-1: none)
+        int64_t n_t = 0, n_a = 0;                          // entries
+        int n_blocks = 0;
+        bool shared = false;  // one set of products serves both sides
+        uint32_t smem = 0;    // dynamic shared memory of the largest block
+    };
+    bool make_resident(DeviceArena& ar, int n_blocks, int esize, int ncv, int nrv, int par_bytes,
+                       uint32_t max_smem, Resident& out) const;
+    // The entries' values from this matrix's values of the same precision.
+    void fill_resident(DeviceArena& ar, Resident& r, bool f32, cudaStream_t s) const;
     // Build and upload A's long rows by column segment (build_seg) and a tiling of
     // their (segment, long row) pairs in stage geometry g, interleaved one block per
     // segment (interleave_tiles); false when no row qualifies.  `is_long` receives

@@ -121,6 +121,122 @@ int32_t build_vec_items(const HostCsr& csr, const std::vector<int32_t>& inst_row
     return slots;
 }
 
+void deal_resident(const HostCsr& csr, const std::vector<int32_t>& inst_row_off, int n_blocks,
+                   HostResident& o) {
+    o = HostResident();
+    const int K = static_cast<int>(inst_row_off.size()) - 1;
+    const std::vector<int32_t>& rp = csr.rp;
+    const int32_t rows = csr.rows;
+    auto lanes_log2 = [](int64_t len) {
+        int lg = 0;
+        while (lg < 5 && (int64_t(1) << lg) * kResLaneNnz < len) ++lg;
+        return lg;
+    };
+    const double total = rows > 0 ? static_cast<double>(rp[rows]) + 4.0 * rows : 0.0;
+    int32_t r = 0;
+    int p = 0;
+    std::vector<int32_t> order;
+    std::vector<ResSlice> sl;   // one block's slices
+    std::vector<int32_t> lr, by;  // their lanes' rows, their order
+    for (int b = 0; b < n_blocks; ++b) {
+        ResBlock B{};
+        B.row0 = r;
+        const double want = total * (b + 1) / n_blocks;
+        while (r < rows && (b + 1 == n_blocks ||
+                            static_cast<double>(rp[r + 1]) + 4.0 * (r + 1) <= want + 0.5)) ++r;
+        B.row1 = r;
+        B.slice0 = static_cast<int32_t>(o.slices.size());
+        B.elem0 = b > 0 ? o.blocks.back().elem0 + o.blocks.back().n_elem : 0;
+        B.long0 = static_cast<int32_t>(o.longs.size());
+        while (p + 1 < K && inst_row_off[p + 1] <= B.row0) ++p;
+        B.inst0 = p;
+        sl.clear();
+        lr.clear();
+        auto add_slice = [&](int depth, int lg, int inst, int slot, int32_t row) {
+            sl.push_back(ResSlice{B.n_elem, depth * 8 + lg, inst, slot});
+            lr.resize(lr.size() + 32, row);
+            B.n_elem += 32 * depth;
+        };
+        int q = p;
+        for (int32_t a = B.row0; a < B.row1;) {  // one instance's rows at a time
+            while (q + 1 < K && inst_row_off[q + 1] <= a) ++q;
+            const int32_t e = std::min(B.row1, inst_row_off[q + 1]);
+            order.resize(e - a);
+            std::iota(order.begin(), order.end(), a);
+            auto longer = [&](int32_t x, int32_t y) { return rp[x + 1] - rp[x] > rp[y + 1] - rp[y]; };
+            if (!std::is_sorted(order.begin(), order.end(), longer))
+                std::stable_sort(order.begin(), order.end(), longer);
+            for (size_t i = 0; i < order.size();) {
+                const int32_t row = order[i], len = rp[row + 1] - rp[row];
+                if (len > kResPiece) {
+                    const int32_t np = (len + kResPiece - 1) / kResPiece;
+                    o.longs.push_back(ResLong{row - B.row0, B.n_slots, np, q - B.inst0});
+                    for (int32_t s = 0; s < np; ++s)
+                        add_slice((std::min(kResPiece, len - s * kResPiece) + 31) / 32, 5, q - B.inst0,
+                                  B.n_slots++, static_cast<int32_t>(o.longs.size()) - 1 - B.long0);
+                    ++i;
+                    continue;
+                }
+                const int lg = lanes_log2(len), G = 1 << lg, per = 32 >> lg;
+                const size_t lane0 = lr.size();
+                add_slice((len + G - 1) / G, lg, q - B.inst0, -1, -1);  // the longest row comes first
+                for (int g = 0; g < per && i < order.size(); ++g, ++i) {
+                    if (lanes_log2(rp[order[i] + 1] - rp[order[i]]) != lg) break;
+                    std::fill_n(lr.begin() + lane0 + g * G, G, order[i] - B.row0);
+                }
+            }
+            a = e;
+        }
+        B.n_inst = B.row1 > B.row0 ? q - B.inst0 + 1 : 0;
+        B.n_slices = static_cast<int32_t>(sl.size());
+        B.n_long = static_cast<int32_t>(o.longs.size()) - B.long0;
+        // deepest slices first, so that the warps' last rounds are the short ones
+        by.resize(sl.size());
+        std::iota(by.begin(), by.end(), 0);
+        std::stable_sort(by.begin(), by.end(), [&](int32_t x, int32_t y) {
+            return (sl[x].shape >> 3) > (sl[y].shape >> 3);
+        });
+        for (int32_t s : by) {
+            o.slices.push_back(sl[s]);
+            o.lane_row.insert(o.lane_row.end(), lr.begin() + size_t(32) * s, lr.begin() + size_t(32) * (s + 1));
+        }
+        o.blocks.push_back(B);
+    }
+}
+
+void fill_resident(const HostCsr& csr, HostResident& o) {
+    const std::vector<int32_t>& rp = csr.rp;
+    const size_t n = o.blocks.empty() ? 0 : static_cast<size_t>(o.blocks.back().elem0) + o.blocks.back().n_elem;
+    o.idx.assign(n, -1);
+    o.src.assign(n, -1);
+    for (const ResBlock& B : o.blocks)
+        for (int32_t s = B.slice0; s < B.slice0 + B.n_slices; ++s) {
+            const ResSlice& m = o.slices[s];
+            const int lg = m.shape & 7, G = 1 << lg;
+            int32_t* const idx = o.idx.data() + B.elem0 + m.off;
+            int32_t* const src = o.src.data() + B.elem0 + m.off;
+            for (int g = 0; g < 32; g += G) {
+                const int32_t ln = o.lane_row[size_t(32) * s + g];
+                if (ln < 0) continue;
+                int32_t k0, k1;
+                if (m.slot >= 0) {
+                    const ResLong& l = o.longs[B.long0 + ln];
+                    const int32_t row = B.row0 + l.row;
+                    k0 = rp[row] + (m.slot - l.slot0) * kResPiece;
+                    k1 = std::min(k0 + kResPiece, rp[row + 1]);
+                } else {
+                    k0 = rp[B.row0 + ln];
+                    k1 = rp[B.row0 + ln + 1];
+                }
+                for (int32_t k = k0; k < k1; ++k) {
+                    const int32_t x = ((k - k0) >> lg) * 32 + g + ((k - k0) & (G - 1));
+                    idx[x] = csr.ci[k];
+                    src[x] = k;
+                }
+            }
+        }
+}
+
 bool build_seg(const HostCsr& csr, const std::vector<int32_t>& inst_row_off, int nseg,
                int long_min, HostSeg& o) {
     o = HostSeg();

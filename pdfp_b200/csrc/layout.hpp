@@ -228,6 +228,97 @@ bool build_seg(const HostCsr& csr, const std::vector<int32_t>& inst_row_off, int
 // are padded with empty tiles of instance -1.
 void interleave_tiles(const HostTiling& in, int nseg, HostTiling& out);
 
+// ---- the resident window (resident_steps.cuh) ------------------------------------
+// One side of the matrix dealt to the blocks of a grid that keeps it in shared memory:
+// block b owns the packed rows [row0, row1), cut into SLICES of 32 lanes.  A slice
+// holds 32 >> lg rows with 2^lg lanes each; lane l's entries are idx[off + u * 32 + l],
+// u = 0 .. depth-1 (index -1: no entry), its row is lane_row[slice * 32 + l] (relative
+// to row0, -1: none).  A row of more than kResPiece nonzeros takes several slices of
+// one row each (slot >= 0: the slice's partial-sum slot; lane_row then holds the row's
+// ResLong in the block's list), whose sums are added in slot order.
+constexpr int kResLaneNnz = 32;  // nonzeros per lane that set a row's lanes (a power of two up to 32)
+constexpr int kResPiece = 1024;  // nonzeros per slice of a long row (32 per lane)
+
+struct alignas(16) ResSlice {
+    int32_t off;    // first entry, relative to the block's entries
+    int32_t shape;  // depth * 8 + lg
+    int32_t inst;   // instance, relative to the block's inst0
+    int32_t slot;   // -1, or the partial-sum slot of a long row's piece
+};
+struct alignas(16) ResLong {
+    int32_t row, slot0, np, inst;  // row relative to row0, instance relative to inst0
+};
+struct alignas(16) ResBlock {
+    int32_t row0, row1, slice0, n_slices;
+    int32_t elem0, n_elem, inst0, n_inst;
+    int32_t long0, n_long, n_slots, pad;
+};
+struct HostResident {
+    std::vector<ResBlock> blocks;
+    std::vector<ResSlice> slices;
+    std::vector<ResLong> longs;
+    std::vector<int32_t> lane_row;  // 32 per slice
+    std::vector<int32_t> idx, src;  // per entry: gathered index and CSR position (-1: none)
+};
+// Deals the rows to n_blocks contiguous ranges of about equal nonzeros + 4 per row.
+// A row's lanes, and with them the order in which its terms are added, depend on its
+// length alone, never on its block.
+// deal_resident makes the blocks, slices and rows (which tell what a block's shared
+// memory must hold), fill_resident then the entries.
+void deal_resident(const HostCsr& csr, const std::vector<int32_t>& inst_row_off, int n_blocks,
+                   HostResident& out);
+void fill_resident(const HostCsr& csr, HostResident& out);
+// Dynamic shared memory a block needs for its share of both sides, with `esize`-byte
+// reals, ncv / nrv vectors kept per column / row and par_bytes of parameters per
+// instance; `shared`: one set of products serves both sides in turn.  The kernel carves
+// its memory with the same function.
+struct ResSmem {
+    uint32_t col, row, val_t, val_a, prod_t, prod_a, par_t, par_a, slots_t, slots_a, idx_t, idx_a, lane_t, lane_a,
+        slice_t, slice_a, long_t, long_a, arr_t, arr_a, total;
+};
+PDFP_HD inline ResSmem res_smem(const ResBlock& t, const ResBlock& a, int esize, int ncv, int nrv,
+                                int par_bytes, bool shared) {
+    ResSmem s;
+    uint32_t off = 0;
+    auto take = [&](uint64_t bytes) {
+        const uint32_t at = off;
+        off += static_cast<uint32_t>((bytes + 15) & ~uint64_t(15));
+        return at;
+    };
+    s.col = take(uint64_t(esize) * ncv * (t.row1 - t.row0));
+    s.row = take(uint64_t(esize) * nrv * (a.row1 - a.row0));
+    s.val_t = take(uint64_t(esize) * t.n_elem);
+    s.val_a = take(uint64_t(esize) * a.n_elem);
+    s.prod_t = take(uint64_t(esize) * (shared && a.n_elem > t.n_elem ? a.n_elem : t.n_elem));
+    s.prod_a = shared ? s.prod_t : take(uint64_t(esize) * a.n_elem);
+    s.par_t = take(uint64_t(par_bytes) * t.n_inst);
+    s.par_a = take(uint64_t(par_bytes) * a.n_inst);
+    s.slots_t = take(uint64_t(8) * t.n_slots);
+    s.slots_a = take(uint64_t(8) * a.n_slots);
+    s.idx_t = take(uint64_t(4) * t.n_elem);
+    s.idx_a = take(uint64_t(4) * a.n_elem);
+    s.lane_t = take(uint64_t(128) * t.n_slices);
+    s.lane_a = take(uint64_t(128) * a.n_slices);
+    s.slice_t = take(uint64_t(16) * t.n_slices);
+    s.slice_a = take(uint64_t(16) * a.n_slices);
+    s.long_t = take(uint64_t(16) * t.n_long);
+    s.long_a = take(uint64_t(16) * a.n_long);
+    s.arr_t = take(uint64_t(4) * t.n_long);
+    s.arr_a = take(uint64_t(4) * a.n_long);
+    s.total = off;
+    return s;
+}
+
+// Device view of one side.
+struct ResDev {
+    const ResBlock* blocks = nullptr;
+    const ResSlice* slices = nullptr;
+    const ResLong* longs = nullptr;
+    const int32_t* lane_row = nullptr;
+    const int32_t* idx = nullptr;
+    const void* val = nullptr;  // values in the precision of the steps, in entry order
+};
+
 // One problem as handed to the library (CSR, caller's numbering).
 struct ProblemIn {
     int32_t m, n;

@@ -26,6 +26,7 @@
 #include "power.cuh"
 #include "tiny_steps.cuh"
 #include "medium_steps.cuh"
+#include "resident_steps.cuh"
 #include "projector.hpp"
 
 namespace pdfp {
@@ -941,6 +942,30 @@ Projector::Projector(const std::vector<ProblemData>& probs, int precision) : pre
             }
         }
     }
+    // A window's steps with the whole handle resident on the chip (resident_steps.cuh),
+    // where it fits and no switch names another form of the steps; PDFP_RESIDENT=0
+    // switches it off.
+    {
+        const char* re = std::getenv("PDFP_RESIDENT");
+        resident_ = !(re && re[0] == '0') && !tiny_ && L.NNZ > 0;
+        for (const char* name : {"PDFP_STEP_ENGINE", "PDFP_TUNING", "PDFP_SEG", "PDFP_MEDIUM", "PDFP_VEC_WINDOW",
+                                 "PDFP_STEP_OVERLAP", "PDFP_STREAM_EVICT_FIRST"})
+            if (std::getenv(name)) resident_ = false;
+    }
+}
+
+// The resident form of precision T, laid out the first time a window or a query asks.
+template <typename T>
+ResidentForm& Projector::ensure_resident() {
+    std::shared_ptr<ResidentForm>& f = std::is_same<T, float>::value ? res32_ : res64_;
+    if (!f) f = std::make_shared<ResidentForm>();
+    if (resident_) f->prepare<PdfpResident<T>>(M_, ar_, num_sms_, max_smem_block_, stream_);
+    return *f;
+}
+
+int32_t Projector::window_form() {
+    if (tiny_ || vecwin_ || medium_ || !resident_) return tiny_ ? 3 : vecwin_ ? 2 : medium_ ? 1 : 0;
+    return (precision_ == PDFP_MIXED ? ensure_resident<float>() : ensure_resident<double>()).ready() ? 4 : 0;
 }
 
 template <>
@@ -1552,6 +1577,13 @@ void Projector::launch_medium_steps(int i0, int i1) {
                                static_cast<int32_t>(i1)));
 }
 
+// Steps i0 .. i1 (i1: a window's last, major) with the handle resident on the chip.
+template <typename T>
+void Projector::launch_resident_steps(int i0, int i1) {
+    const int mode = std::is_same<T, float>::value ? MODE_FP32 : MODE_FP64;
+    ensure_resident<T>().launch(PdfpResident<T>{vecs<T>(), st_, M_.row_off, M_.n_eq, mode, err_}, K_, i0, i1, stream_);
+}
+
 void Projector::launch_vec_window(int i0, int i1) {
     using POp = PrimalOp<float, false, kFlatThreads>;
     using DOp = DualOp<float, false, kFlatThreads>;
@@ -1647,6 +1679,15 @@ void Projector::record_window(int freq, bool with32, bool with64) {
             launch_vec_window(2, freq);
             after_step = false;
             i = freq - 1;
+            continue;
+        }
+        if (!sample && i == 2 && (!with32 || ensure_resident<float>().ready()) &&
+            (!with64 || ensure_resident<double>().ready())) {
+            // steps 2 .. freq in one cooperative launch per precision
+            if (with32) launch_resident_steps<float>(2, freq);
+            if (with64) launch_resident_steps<double>(2, freq);
+            after_step = false;
+            i = freq;
             continue;
         }
         if (medium_ && !sample && i == 2 && freq > 2) {
@@ -1768,6 +1809,8 @@ cudaGraphExec_t Projector::window_graph(int freq, bool with32, bool with64) {
     auto it = graphs_.find(key);
     if (it != graphs_.end()) return it->second;
     prepare_window();
+    if (with32) ensure_resident<float>();
+    if (with64) ensure_resident<double>();
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     PDFP_CK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));

@@ -61,6 +61,48 @@ __device__ __forceinline__ StepParams<T> step_params(const InstState& st, int32_
     return p;
 }
 
+// primal_step! and dual_y_step! of one column (src/pdfp.jl:119-143): pv = {x, x0, y, y0,
+// l, u, x~, w} (w < 0 marks a column outside I), sum = (A'z)_j.
+template <typename T>
+struct PrimalCell {
+    T cx, rx, cy;          // the new iterates and x_bar
+    T px, t, py, ry;       // x_hat, its unclamped argument, y_hat, reflected y (major steps)
+};
+template <typename T>
+__device__ __forceinline__ PrimalCell<T> primal_cell(const StepParams<T>& p, const T (&pv)[8], T sum) {
+    const T cx = pv[0], ix = pv[1], cy = pv[2], iy = pv[3];
+    const T lb = pv[4], ub = pv[5], xt = pv[6], w = pv[7];
+    PrimalCell<T> o;
+    // primal_step!  (src/pdfp.jl:124-129)
+    o.t = sub_rn(cx, mul_rn(p.tau, sub_rn(sum, cy)));
+    o.px = jl_clamp(o.t, lb, ub);
+    o.rx = sub_rn(mul_rn(T(2), o.px), cx);
+    o.cx = halpern(p.weight, p.omega, p.omw, p.omwt, o.rx, cx, ix);
+    // dual_y_step!  (src/pdfp.jl:138-141); w < 0 marks j outside I
+    o.py = w >= T(0) ? jl_clamp(add_rn(cy, mul_rn(p.sigma, sub_rn(xt, o.rx))), -w, w) : T(0);
+    o.ry = sub_rn(mul_rn(T(2), o.py), cy);
+    o.cy = halpern(p.weight, p.omega, p.omw, p.omwt, o.ry, cy, iy);
+    return o;
+}
+
+// dual_z_step! of one row (src/pdfp.jl:146-156): pv = {z, z0, b}, sum = (A x_bar)_i.
+template <typename T>
+struct DualCell {
+    T cz;      // the new iterate
+    T pz, rz;  // z_hat and its reflection (major steps)
+};
+template <typename T>
+__device__ __forceinline__ DualCell<T> dual_cell(const StepParams<T>& p, bool eq, const T (&pv)[3], T sum) {
+    const T cz = pv[0], iz = pv[1], b = pv[2];
+    DualCell<T> o;
+    // dual_z_step!  (src/pdfp.jl:150-154)
+    const T raw = add_rn(cz, mul_rn(p.sigma, sub_rn(sum, b)));
+    o.pz = eq ? raw : jl_max(raw, T(0));
+    o.rz = sub_rn(mul_rn(T(2), o.pz), cz);
+    o.cz = halpern(p.weight, p.omega, p.omw, p.omwt, o.rz, cz, iz);
+    return o;
+}
+
 // ---- the PDHG step ------------------------------------------------------------
 
 template <typename T, bool MAJOR, int NTHREADS>
@@ -114,23 +156,15 @@ struct PrimalOp {
     }
     // The epilogue on column j's inputs pv (staged() order) and its sum s = (A'z)_j.
     __device__ void row_vals(int32_t j, const TileP& p, const T (&pv)[NVEC], const T (&s)[1]) const {
-        const T cx = pv[0], ix = pv[1], cy = pv[2], iy = pv[3];
-        const T lb = pv[4], ub = pv[5], xt = pv[6], w = pv[7];
-        // primal_step!  (src/pdfp.jl:124-129)
-        const T t = sub_rn(cx, mul_rn(p.tau, sub_rn(s[0], cy)));
-        const T xh = jl_clamp(t, lb, ub);
-        const T rx = sub_rn(mul_rn(T(2), xh), cx);
-        v.cx[j] = halpern(p.weight, p.omega, p.omw, p.omwt, rx, cx, ix);
-        v.rx[j] = rx;
-        // dual_y_step!  (src/pdfp.jl:138-141); w < 0 marks j outside I
-        const T yh = w >= T(0) ? jl_clamp(add_rn(cy, mul_rn(p.sigma, sub_rn(xt, rx))), -w, w) : T(0);
-        const T ry = sub_rn(mul_rn(T(2), yh), cy);
-        v.cy[j] = halpern(p.weight, p.omega, p.omw, p.omwt, ry, cy, iy);
+        const PrimalCell<T> o = primal_cell(p, pv, s[0]);
+        v.cx[j] = o.cx;
+        v.rx[j] = o.rx;
+        v.cy[j] = o.cy;
         if (MAJOR) {
-            v.px[j] = xh;
-            v.ds[j] = sub_rn(xh, t) / p.tau;
-            v.py[j] = yh;
-            v.ry[j] = ry;
+            v.px[j] = o.px;
+            v.ds[j] = sub_rn(o.px, o.t) / p.tau;
+            v.py[j] = o.py;
+            v.ry[j] = o.ry;
         }
     }
 };
@@ -184,15 +218,11 @@ struct DualOp {
     }
     // The epilogue on row i's inputs pv (staged() order) and its sum s = (A x_bar)_i.
     __device__ void row_vals(int32_t i, const TileP& t, const T (&pv)[NVEC], const T (&s)[1]) const {
-        const T cz = pv[0], iz = pv[1], b = pv[2];
-        // dual_z_step!  (src/pdfp.jl:150-154)
-        const T raw = add_rn(cz, mul_rn(t.p.sigma, sub_rn(s[0], b)));
-        const T zh = i < t.eq_end ? raw : jl_max(raw, T(0));
-        const T rz = sub_rn(mul_rn(T(2), zh), cz);
-        v.cz[i] = halpern(t.p.weight, t.p.omega, t.p.omw, t.p.omwt, rz, cz, iz);
+        const DualCell<T> o = dual_cell(t.p, i < t.eq_end, pv, s[0]);
+        v.cz[i] = o.cz;
         if (MAJOR) {
-            v.pz[i] = zh;
-            v.rz[i] = rz;
+            v.pz[i] = o.pz;
+            v.rz[i] = o.rz;
         }
     }
 };

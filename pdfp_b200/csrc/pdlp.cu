@@ -18,6 +18,7 @@
 #include "device.hpp"
 #include "kernels.cuh"
 #include "pdlp_ops.cuh"
+#include "resident_steps.cuh"
 #include "tiny_steps.cuh"
 #include "power.cuh"
 #include "solvers.hpp"
@@ -601,6 +602,11 @@ class LpSolver {
     const DeviceMatrix::Tiling& tiling_a() const {
         return (std::is_same<T, double>::value && f32_) ? it64_a_ : it_a_;
     }
+    ResidentForm res32_, res64_;  // the window's steps with the LP on the chip, where it fits
+    template <typename T>
+    ResidentForm& resident() {
+        return std::is_same<T, float>::value ? res32_ : res64_;
+    }
     template <typename T>
     cudaGraphExec_t build_graph(int freq);
 };
@@ -651,10 +657,13 @@ void LpSolver::record(int freq) {
                                               M_.rp_t, M_.ci_t, M_.rp_a, M_.ci_a, M_.col_off,
                                               M_.row_off, 2, freq);
         PDFP_CK(cudaGetLastError());
+        step(freq, true);
+    } else if (resident<T>().ready()) {  // steps 2 .. freq with the LP resident on the chip
+        resident<T>().launch(LpResident<T>{v, st_, mode, err_}, 1, 2, freq, stream_);
     } else {
         for (int i = 2; i <= freq - 1; ++i) step(i, false);
+        step(freq, true);
     }
-    step(freq, true);
     evals(EVAL_FULL);
     if (cupdlpx_) {
         zero_maxes_kernel<<<1, 32, 0, stream_>>>(d_.maxes);
@@ -693,6 +702,10 @@ void LpSolver::launch_tiny_solve() {
 template <typename T>
 cudaGraphExec_t LpSolver::build_graph(int freq) {
     prepare_grids<T>();
+    {
+        const char* re = std::getenv("PDFP_RESIDENT");
+        if (!(re && re[0] == '0') && !tiny_) resident<T>().template prepare<LpResident<T>>(M_, ar_, sms_, max_smem_, stream_);
+    }
     cudaGraph_t g = nullptr;
     cudaGraphExec_t exec = nullptr;
     PDFP_CK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));

@@ -42,6 +42,40 @@ __device__ __forceinline__ void atomic_max_nonneg(unsigned long long* slot, doub
     atomicMax(slot, static_cast<unsigned long long>(__double_as_longlong(v)));
 }
 
+// primal_step! of one column (src/pdlp.jl:115-132; tau is the primal step): pv = {x, x0,
+// c, l, u}, sum = (A'y)_j.
+template <typename T>
+struct LpPrimalCell {
+    T cx, rx, px, t;  // the new iterate, x_bar, x_hat and its unclamped argument
+};
+template <typename T>
+__device__ __forceinline__ LpPrimalCell<T> lp_primal_cell(const StepParams<T>& p, const T (&pv)[5], T sum) {
+    const T cx = pv[0], ix = pv[1], c = pv[2], lb = pv[3], ub = pv[4];
+    LpPrimalCell<T> o;
+    o.t = sub_rn(cx, mul_rn(p.tau, sub_rn(c, sum)));
+    o.px = jl_clamp(o.t, lb, ub);
+    o.rx = sub_rn(mul_rn(T(2), o.px), cx);
+    o.cx = halpern(p.weight, p.omega, p.omw, p.omwt, o.rx, cx, ix);
+    return o;
+}
+
+// dual_step! of one row (src/pdlp.jl:134-145; sigma is the dual step): pv = {y, y0, lower,
+// upper}, sum = (A x_bar)_i.
+template <typename T>
+struct LpDualCell {
+    T cy, py, ry;  // the new iterate, y_hat and its reflection
+};
+template <typename T>
+__device__ __forceinline__ LpDualCell<T> lp_dual_cell(const StepParams<T>& p, const T (&pv)[4], T sum) {
+    const T cy = pv[0], iy = pv[1], clb = pv[2], cub = pv[3];
+    LpDualCell<T> o;
+    const T t = sub_rn(cy / p.sigma, sum);
+    o.py = mul_rn(sub_rn(t, jl_clamp(t, -cub, -clb)), p.sigma);
+    o.ry = sub_rn(mul_rn(T(2), o.py), cy);
+    o.cy = halpern(p.weight, p.omega, p.omw, p.omwt, o.ry, cy, iy);
+    return o;
+}
+
 template <typename T, bool MAJOR, int NTHREADS>
 struct LpPrimalOp {
     using MT = T;
@@ -66,15 +100,12 @@ struct LpPrimalOp {
     __device__ void gather(int32_t col, T (&g)[1]) const { g[0] = v.cy[col]; }
     __device__ void row(int32_t j, int32_t rr, int, const TileP& p, const T* const* sv,
                         const T (&s)[1], double*) const {
-        const T cx = sv[0][rr], ix = sv[1][rr], c = sv[2][rr], lb = sv[3][rr], ub = sv[4][rr];
-        // primal_step!, src/pdlp.jl:115-132 (tau is the primal step here)
-        const T t = sub_rn(cx, mul_rn(p.tau, sub_rn(c, s[0])));
-        const T xh = jl_clamp(t, lb, ub);
-        if (MAJOR) v.ds[j] = sub_rn(xh, t) / p.tau;
-        v.px[j] = xh;
-        const T rx = sub_rn(mul_rn(T(2), xh), cx);
-        v.rx[j] = rx;
-        v.cx[j] = halpern(p.weight, p.omega, p.omw, p.omwt, rx, cx, ix);
+        const T pv[5] = {sv[0][rr], sv[1][rr], sv[2][rr], sv[3][rr], sv[4][rr]};
+        const LpPrimalCell<T> o = lp_primal_cell(p, pv, s[0]);
+        if (MAJOR) v.ds[j] = sub_rn(o.px, o.t) / p.tau;
+        v.px[j] = o.px;
+        v.rx[j] = o.rx;
+        v.cx[j] = o.cx;
     }
     __device__ void write_partials(int32_t, const double*) const {}
 };
@@ -103,16 +134,59 @@ struct LpDualOp {
     __device__ void gather(int32_t col, T (&g)[1]) const { g[0] = v.rx[col]; }
     __device__ void row(int32_t i, int32_t rr, int, const TileP& p, const T* const* sv,
                         const T (&s)[1], double*) const {
-        const T cy = sv[0][rr], iy = sv[1][rr], clb = sv[2][rr], cub = sv[3][rr];
-        // dual_step!, src/pdlp.jl:134-145 (sigma is the dual step here)
-        const T t = sub_rn(cy / p.sigma, s[0]);
-        const T yh = mul_rn(sub_rn(t, jl_clamp(t, -cub, -clb)), p.sigma);
-        if (MAJOR) v.py[i] = yh;
-        const T ry = sub_rn(mul_rn(T(2), yh), cy);
-        v.ry[i] = ry;
-        v.cy[i] = halpern(p.weight, p.omega, p.omw, p.omwt, ry, cy, iy);
+        const T pv[4] = {sv[0][rr], sv[1][rr], sv[2][rr], sv[3][rr]};
+        const LpDualCell<T> o = lp_dual_cell(p, pv, s[0]);
+        if (MAJOR) v.py[i] = o.py;
+        v.ry[i] = o.ry;
+        v.cy[i] = o.cy;
     }
     __device__ void write_partials(int32_t, const double*) const {}
+};
+
+// The steps as the resident window runs them (resident_steps.cuh).
+template <typename TT>
+struct LpResident {
+    using T = TT;
+    static constexpr int NCV = 5, NRV = 4;
+    LpVecs<T> v;
+    const InstState* st;
+    int32_t mode;
+    int32_t* errp;
+    __device__ bool active(int p) const { return st[p].status == ST_RUNNING && st[p].mode == mode; }
+    __device__ int32_t eq_end(int) const { return 0; }
+    __device__ T* col_vec(int q) const {
+        T* const s[NCV] = {v.cx, v.ix, v.c, v.lb, v.ub};
+        return s[q];
+    }
+    __device__ T* row_vec(int q) const {
+        T* const s[NRV] = {v.cy, v.iy, v.clb, v.cub};
+        return s[q];
+    }
+    template <bool MAJOR>
+    __device__ __forceinline__ T col(const StepParams<T>& p, int32_t j, const T (&in)[NCV], T* pv, int,
+                                     T sum) const {
+        const LpPrimalCell<T> o = lp_primal_cell(p, in, sum);
+        pv[0] = o.cx;
+        if (MAJOR) {
+            v.ds[j] = sub_rn(o.px, o.t) / p.tau;
+            v.px[j] = o.px;
+            v.rx[j] = o.rx;
+        }
+        return o.rx;
+    }
+    template <bool MAJOR>
+    __device__ __forceinline__ T row(const StepParams<T>& p, bool, int32_t i, const T (&in)[NRV], T* pv, int,
+                                     T sum) const {
+        const LpDualCell<T> o = lp_dual_cell(p, in, sum);
+        pv[0] = o.cy;
+        if (MAJOR) {
+            v.py[i] = o.py;
+            v.ry[i] = o.ry;
+        }
+        return o.cy;
+    }
+    __device__ static bool col_changes(int q) { return q == 0; }
+    __device__ static bool row_changes(int q) { return q == 0; }
 };
 
 // Column terms: A'y_hat and A'(y_hat - y_bar) in one pass over A'.

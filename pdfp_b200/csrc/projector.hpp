@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <map>
+#include <memory>
 #include <set>
 #include <vector>
 
@@ -12,6 +13,8 @@
 #include "state.hpp"
 
 namespace pdfp {
+
+struct ResidentForm;  // resident_steps.cuh
 
 // One projection problem in the caller's numbering (scaled data).
 struct ProblemData {
@@ -69,8 +72,9 @@ class Projector {
     // {segments, long-row threshold}, {0, 0} when it has none.
     void tuning_seg(int32_t* out) const;
     // 0: per-step launches (graph), 1: cooperative row passes, 2: cooperative vec
-    // window, 3: whole windows per small member in one launch
-    int32_t window_form() const { return tiny_ ? 3 : vecwin_ ? 2 : medium_ ? 1 : 0; }
+    // window, 3: whole windows per small member in one launch, 4: the handle resident on
+    // the chip for a window's steps
+    int32_t window_form();
     // Every autotuner measurement: ms[i] and cfg[7i..7i+6] = {side (0: A', 1: A),
     // stage bytes, gatherer threads, gather policy, stages, blocks per SM cap,
     // reducer threads}; side 2: the A side with its long rows by column segment,
@@ -140,6 +144,10 @@ class Projector {
     void launch_tiny_steps(int i0, int i1);
     template <typename T>
     void launch_medium_steps(int i0, int i1);
+    template <typename T>
+    void launch_resident_steps(int i0, int i1);
+    template <typename T>
+    ResidentForm& ensure_resident();
     cudaGraphExec_t window_graph(int freq, bool with32, bool with64);
     void prepare_window();
     void run_window(int freq, bool with32, bool with64);
@@ -203,6 +211,10 @@ class Projector {
     bool medium_ = false;  // a mid-sized handle: the minor steps in one cooperative launch
     int32_t *part_t_ = nullptr, *part_a_ = nullptr;  // each block's rows of A' and of A
     unsigned* gbar_ = nullptr;                          // the grid barrier's words
+    // Whether a window's steps may run with the whole handle resident on the chip, and
+    // each precision's form once a window needed it.
+    bool resident_ = false;
+    std::shared_ptr<ResidentForm> res32_, res64_;
     bool vecwin_ = false;  // FP32 minor steps of a window in one cooperative vec launch
     int vecwin_grid_ = 0;  // its blocks (all resident)
     void launch_vec_window(int i0, int i1);

@@ -1,0 +1,154 @@
+"""The resident window (resident_steps.cuh): a window's steps in one cooperative launch
+with the whole handle in shared memory.
+
+CPU: tests/native/resident_check.cpp walks the layout with the kernel's index arithmetic.
+GPU: the steps against the per-step launches (PDFP_RESIDENT=0) and the FP64 oracle, and a
+batch's members against their single handles, bit for bit."""
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+import scipy.sparse as sp
+
+from pdfp_b200 import synthetic
+from pdfp_b200.params import SolverParameters
+from test_layout import rand_csr
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+ROOT = os.path.dirname(HERE)
+OUT = os.path.join(ROOT, "_build", "libresident_check.so")
+
+
+@pytest.fixture(scope="module")
+def checker():
+    os.makedirs(os.path.dirname(OUT), exist_ok=True)
+    srcs = [os.path.join(HERE, "native", "resident_check.cpp"),
+            os.path.join(ROOT, "pdfp_b200", "csrc", "layout.cpp")]
+    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-o", OUT] + srcs, check=True)
+    lib = C.CDLL(OUT)
+    lib.resident_check.restype = C.c_int
+    return lib
+
+
+def check(lib, mats, eqs, n_blocks):
+    K = len(mats)
+    keep = []
+    ms, ns = (C.c_int32 * K)(), (C.c_int32 * K)()
+    rps, cis = (C.POINTER(C.c_int32) * K)(), (C.POINTER(C.c_int32) * K)()
+    vs, es = (C.POINTER(C.c_double) * K)(), (C.POINTER(C.c_uint8) * K)()
+    for p, (A, e) in enumerate(zip(mats, eqs)):
+        A = sp.csr_matrix(A)
+        A.sort_indices()
+        rp = np.ascontiguousarray(A.indptr, dtype=np.int32)
+        ci = np.ascontiguousarray(A.indices if A.nnz else np.zeros(1), dtype=np.int32)
+        v = np.ascontiguousarray(A.data if A.nnz else np.zeros(1), dtype=np.float64)
+        ee = np.ascontiguousarray(e, dtype=np.uint8) if len(e) else np.zeros(1, np.uint8)
+        keep += [rp, ci, v, ee]
+        ms[p], ns[p] = A.shape
+        rps[p] = rp.ctypes.data_as(C.POINTER(C.c_int32))
+        cis[p] = ci.ctypes.data_as(C.POINTER(C.c_int32))
+        vs[p] = v.ctypes.data_as(C.POINTER(C.c_double))
+        es[p] = ee.ctypes.data_as(C.POINTER(C.c_uint8))
+    stats = (C.c_int64 * 2)()
+    return lib.resident_check(K, ms, ns, rps, cis, vs, es, n_blocks, stats), list(stats)
+
+
+@pytest.mark.parametrize("n_blocks", [1, 7, 148])
+def test_layout(checker, n_blocks):
+    rng = np.random.default_rng(5)
+    one = [rand_csr(rng, 300, 500, 0.02)]
+    long = [rand_csr(rng, 60, 9000, 0.0005, long_rows=4, long_len=7001)]
+    # row lengths at the edges of the lanes' rule and of a long row's pieces
+    edges = [0, 1, 31, 32, 33, 64, 65, 128, 129, 256, 257, 512, 513, 1023, 1024, 1025, 2048, 2049]
+    E = sp.lil_matrix((len(edges), 2100))
+    for i, k in enumerate(edges):
+        E[i, rng.choice(2100, size=k, replace=False)] = 1.0
+    batch = [rand_csr(rng, 80, 60, 0.05), sp.csr_matrix((0, 5)), sp.csr_matrix((7, 0)),
+             sp.csr_matrix((4, 6)), rand_csr(rng, 1000, 30, 0.3), sp.csr_matrix(E)]
+    for mats, has_long in ((one, False), (long, True), ([sp.csr_matrix(E)], True), (batch, True)):
+        rc, stats = check(checker, mats, [rng.random(A.shape[0]) < 0.5 for A in mats], n_blocks)
+        assert rc == 0
+        assert (stats[1] > 0) == has_long
+
+
+def _state(probs, precision, monkeypatch, resident):
+    from pdfp_b200 import gpu
+    monkeypatch.setenv("PDFP_RESIDENT", resident)
+    s = gpu.PDFPState(*probs, precision=precision)
+    form = gpu.C.c_int32()
+    gpu.L.check(gpu.L.lib().pdfp_get_window_form(s._h, gpu.C.byref(form)))
+    assert form.value == (4 if resident == "1" else 0)
+    return s
+
+
+def _models():
+    """Ragged general model (no size a multiple of a warp or of the SM count), equality
+    rows among them; Zipf rows long enough for several pieces; binary covering."""
+    g, _, xt = synthetic.general_integer(3, m=1501, n=4013, m_eq=377, mean_row=9.0)
+    z, _ = synthetic.zipf_lp(2, m=3001, n=6007, nnz=60_001)
+    rng = np.random.default_rng(4)
+    zt = np.zeros(6007)
+    zt[z.int_idx] = np.round(rng.random(len(z.int_idx)))
+    return [("general", g, xt), ("zipf", z, zt)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("which", [0, 1])
+def test_steps_match_per_step_launches_and_oracle(oracle, monkeypatch, precision, which):
+    """One and three windows.  FP64: both forms stay within 1e-10 of the oracle after 200
+    and 600 steps (each step adds rounding of about 1e-16 relative and does not expand it);
+    mixed: within 2e-4 of it, FP32 rounding grown by the same argument."""
+    _, milp, xt = _models()[which]
+    sc, is_eq, is_int, w = oracle.projector_inputs(milp)
+    probs = (sc.A, sc.con_ub, is_eq, is_int, sc.var_lb, sc.var_ub, w)
+    for windows in (1, 3):
+        prm = SolverParameters(eps_optimal_relative=1e-9, eps_feasible_relative=1e-9,
+                               iteration_limit=200 * windows)
+        o = oracle.OracleSolvers.PDFPState(*probs)
+        o.set_target(xt / sc.D_c)
+        o.solve(prm, 1.0)
+        tol = 1e-10 if precision == "fp64" else 2e-4
+        for resident in ("1", "0"):
+            s = _state(probs, precision, monkeypatch, resident)
+            s.set_target(xt / sc.D_c)
+            s.solve(prm, 1.0)
+            assert s.total_count == 200 * windows
+            for name in ("pdhg_x", "pdhg_y", "pdhg_z", "current_x", "current_y", "current_z", "dual_slack"):
+                a, b = s.get(name), o.get(name)
+                assert np.linalg.norm(a - b) <= tol * max(1.0, np.linalg.norm(b)), (resident, windows, name)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_batch_members_equal_single_handles(oracle, monkeypatch, precision):
+    """Members that stop at different windows, one of them with long rows: with the same
+    kernels for the windows' first steps (PDFP_AUTOTUNE=0), the steps of the single
+    handles bit for bit in the resident part; whole solves to 1e-12 / 1e-5."""
+    from pdfp_b200 import gpu
+    monkeypatch.setenv("PDFP_RESIDENT", "1")
+    monkeypatch.setenv("PDFP_AUTOTUNE", "0")
+    models = synthetic.covering_packing_batch(seed=7, k=4, n_min=3000, n_max=9000)
+    models.append(_models()[1][1])
+    rng = np.random.default_rng(21)
+    probs, targets = [], []
+    for m in models:
+        sc, is_eq, is_int, w = oracle.projector_inputs(m)
+        probs.append((sc.A, sc.con_ub, is_eq, is_int, sc.var_lb, sc.var_ub, w))
+        targets.append(np.round(rng.random(len(m.c))) / sc.D_c)
+    prm = [SolverParameters(eps_optimal_relative=1e-9, eps_feasible_relative=1e-9,
+                            iteration_limit=200 * (1 + p % 3)) for p in range(len(models))]
+    b = gpu.PDFPBatch(probs, precision=precision)
+    for p, xt in enumerate(targets):
+        b.set_target(p, xt)
+    b.solve(prm, 1.0)
+    tol = 1e-12 if precision == "fp64" else 1e-5
+    for p, pr in enumerate(probs):
+        s = gpu.PDFPState(*pr, precision=precision)
+        s.set_target(targets[p])
+        s.solve(prm[p], 1.0)
+        assert s.total_count == b.results[p]["total_count"] == 200 * (1 + p % 3)
+        x, y = s.pdhg_x, b.get(p, "pdhg_x")
+        assert np.linalg.norm(x - y) <= tol * max(1.0, np.linalg.norm(x)), p
