@@ -264,8 +264,8 @@ bool DeviceMatrix::make_resident(DeviceArena& ar, int n_blocks, int esize, int n
                          static_cast<double>(esize * ncv + 4) * L.N + static_cast<double>(esize * nrv + 4) * L.M;
     if (n_blocks <= 0 || least > static_cast<double>(n_blocks) * max_smem) return false;
     HostResident ht, ha;
-    deal_resident(L.At, L.col_off, n_blocks, ht);
-    deal_resident(L.A, L.row_off, n_blocks, ha);
+    deal_resident(L.At, L.col_off, n_blocks, kResLaneNnz, 1, false, ht);
+    deal_resident(L.A, L.row_off, n_blocks, kResLaneNnz, 1, false, ha);
     for (int shared = 0; shared < 2 && (shared == 0 || r.smem > max_smem); ++shared) {
         r.smem = 0;
         r.shared = shared != 0;
@@ -273,8 +273,33 @@ bool DeviceMatrix::make_resident(DeviceArena& ar, int n_blocks, int esize, int n
             r.smem = std::max(r.smem, res_smem(ht.blocks[b], ha.blocks[b], esize, ncv, nrv, par_bytes, r.shared).total);
     }
     if (r.smem > max_smem) return false;
-    ::pdfp::fill_resident(L.At, ht);
-    ::pdfp::fill_resident(L.A, ha);
+    upload_resident(ar, ht, ha, kResLaneNnz, r);
+    return true;
+}
+
+bool DeviceMatrix::make_cluster(DeviceArena& ar, int c, int esize, int max_warps, uint32_t max_smem,
+                                Resident& r, int& n_warps) const {
+    r = Resident();
+    HostResident ht, ha;
+    deal_resident(L.At, L.col_off, c, kCluLaneNnz, kCluDepthUnit, true, ht);
+    deal_resident(L.A, L.row_off, c, kCluLaneNnz, kCluDepthUnit, true, ha);
+    if (!ht.longs.empty() || !ha.longs.empty()) return false;
+    for (size_t b = 0; b < ht.blocks.size(); ++b) {
+        const int p = static_cast<int>(b) / c;
+        n_warps = std::max(b == 0 ? 1 : n_warps, ht.blocks[b].n_slices + ha.blocks[b].n_slices);
+        if (n_warps > max_warps) return false;
+        r.smem = std::max(r.smem, clu_smem(ht.blocks[b], ha.blocks[b], esize, L.col_off[p + 1] - L.col_off[p],
+                                           L.row_off[p + 1] - L.row_off[p]).total);
+    }
+    if (r.smem > max_smem) return false;
+    upload_resident(ar, ht, ha, kCluLaneNnz, r);
+    return true;
+}
+
+void DeviceMatrix::upload_resident(DeviceArena& ar, HostResident& ht, HostResident& ha, int lane_nnz,
+                                   Resident& r) const {
+    ::pdfp::fill_resident(L.At, lane_nnz, ht);
+    ::pdfp::fill_resident(L.A, lane_nnz, ha);
     const std::vector<void*> d = ar.upload_group(
         {part(ht.blocks), part(ht.slices), part(ht.longs), part(ht.lane_row), part(ht.idx), part(ht.src),
          part(ha.blocks), part(ha.slices), part(ha.longs), part(ha.lane_row), part(ha.idx), part(ha.src)});
@@ -293,8 +318,10 @@ bool DeviceMatrix::make_resident(DeviceArena& ar, int n_blocks, int esize, int n
     r.src_a = static_cast<const int32_t*>(d[11]);
     r.n_t = static_cast<int64_t>(ht.src.size());
     r.n_a = static_cast<int64_t>(ha.src.size());
-    r.n_blocks = n_blocks;
-    return true;
+    r.n_blocks = static_cast<int>(ht.blocks.size());
+    // the copies from pageable memory may still be under way on the default stream, which
+    // the handle's own stream does not wait for
+    PDFP_CK(cudaStreamSynchronize(0));
 }
 
 template <typename T>

@@ -189,8 +189,17 @@ class DeviceMatrix {
     };
     bool make_resident(DeviceArena& ar, int n_blocks, int esize, int ncv, int nrv, int par_bytes,
                        uint32_t max_smem, Resident& out) const;
+    // The same for whole members in clusters of c blocks each (cluster_windows.cuh): false
+    // when a block would have more slices than warps, a row longer than a slice or more
+    // than max_smem bytes of shared memory; n_warps: the most slices of a block.
+    bool make_cluster(DeviceArena& ar, int c, int esize, int max_warps, uint32_t max_smem, Resident& out,
+                      int& n_warps) const;
     // The entries' values from this matrix's values of the same precision.
     void fill_resident(DeviceArena& ar, Resident& r, bool f32, cudaStream_t s) const;
+  private:
+    void upload_resident(DeviceArena& ar, HostResident& t, HostResident& a, int lane_nnz, Resident& r) const;
+
+  public:
     // Build and upload A's long rows by column segment (build_seg) and a tiling of
     // their (segment, long row) pairs in stage geometry g, interleaved one block per
     // segment (interleave_tiles); false when no row qualifies.  `is_long` receives

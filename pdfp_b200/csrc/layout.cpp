@@ -121,29 +121,34 @@ int32_t build_vec_items(const HostCsr& csr, const std::vector<int32_t>& inst_row
     return slots;
 }
 
-void deal_resident(const HostCsr& csr, const std::vector<int32_t>& inst_row_off, int n_blocks,
-                   HostResident& o) {
+void deal_resident(const HostCsr& csr, const std::vector<int32_t>& inst_row_off, int n_blocks, int lane_nnz,
+                   int depth_unit, bool per_member, HostResident& o) {
     o = HostResident();
     const int K = static_cast<int>(inst_row_off.size()) - 1;
     const std::vector<int32_t>& rp = csr.rp;
     const int32_t rows = csr.rows;
-    auto lanes_log2 = [](int64_t len) {
+    const double per_row = per_member ? 64.0 : 4.0;
+    const int32_t piece = 32 * lane_nnz;  // nonzeros per slice of a long row
+    auto lanes_log2 = [&](int64_t len) {
         int lg = 0;
-        while (lg < 5 && (int64_t(1) << lg) * kResLaneNnz < len) ++lg;
+        while (lg < 5 && (int64_t(1) << lg) * lane_nnz < len) ++lg;
         return lg;
     };
-    const double total = rows > 0 ? static_cast<double>(rp[rows]) + 4.0 * rows : 0.0;
     int32_t r = 0;
     int p = 0;
     std::vector<int32_t> order;
     std::vector<ResSlice> sl;   // one block's slices
     std::vector<int32_t> lr, by;  // their lanes' rows, their order
-    for (int b = 0; b < n_blocks; ++b) {
+    for (int b = 0; b < (per_member ? K : 1) * n_blocks; ++b) {
+        // the rows [lo, hi) are dealt to n_blocks blocks, of which this is number `nth`
+        const int32_t lo = per_member ? inst_row_off[b / n_blocks] : 0;
+        const int32_t hi = per_member ? inst_row_off[b / n_blocks + 1] : rows;
+        const int nth = b % n_blocks;
         ResBlock B{};
         B.row0 = r;
-        const double want = total * (b + 1) / n_blocks;
-        while (r < rows && (b + 1 == n_blocks ||
-                            static_cast<double>(rp[r + 1]) + 4.0 * (r + 1) <= want + 0.5)) ++r;
+        const double want = hi > lo ? (static_cast<double>(rp[hi]) - rp[lo] + per_row * (hi - lo)) * (nth + 1) / n_blocks : 0.0;
+        while (r < hi && (nth + 1 == n_blocks ||
+                          static_cast<double>(rp[r + 1]) - rp[lo] + per_row * (r + 1 - lo) <= want + 0.5)) ++r;
         B.row1 = r;
         B.slice0 = static_cast<int32_t>(o.slices.size());
         B.elem0 = b > 0 ? o.blocks.back().elem0 + o.blocks.back().n_elem : 0;
@@ -153,6 +158,7 @@ void deal_resident(const HostCsr& csr, const std::vector<int32_t>& inst_row_off,
         sl.clear();
         lr.clear();
         auto add_slice = [&](int depth, int lg, int inst, int slot, int32_t row) {
+            depth = (depth + depth_unit - 1) / depth_unit * depth_unit;
             sl.push_back(ResSlice{B.n_elem, depth * 8 + lg, inst, slot});
             lr.resize(lr.size() + 32, row);
             B.n_elem += 32 * depth;
@@ -168,11 +174,11 @@ void deal_resident(const HostCsr& csr, const std::vector<int32_t>& inst_row_off,
                 std::stable_sort(order.begin(), order.end(), longer);
             for (size_t i = 0; i < order.size();) {
                 const int32_t row = order[i], len = rp[row + 1] - rp[row];
-                if (len > kResPiece) {
-                    const int32_t np = (len + kResPiece - 1) / kResPiece;
+                if (len > piece) {
+                    const int32_t np = (len + piece - 1) / piece;
                     o.longs.push_back(ResLong{row - B.row0, B.n_slots, np, q - B.inst0});
                     for (int32_t s = 0; s < np; ++s)
-                        add_slice((std::min(kResPiece, len - s * kResPiece) + 31) / 32, 5, q - B.inst0,
+                        add_slice((std::min(piece, len - s * piece) + 31) / 32, 5, q - B.inst0,
                                   B.n_slots++, static_cast<int32_t>(o.longs.size()) - 1 - B.long0);
                     ++i;
                     continue;
@@ -204,8 +210,9 @@ void deal_resident(const HostCsr& csr, const std::vector<int32_t>& inst_row_off,
     }
 }
 
-void fill_resident(const HostCsr& csr, HostResident& o) {
+void fill_resident(const HostCsr& csr, int lane_nnz, HostResident& o) {
     const std::vector<int32_t>& rp = csr.rp;
+    const int32_t piece = 32 * lane_nnz;
     const size_t n = o.blocks.empty() ? 0 : static_cast<size_t>(o.blocks.back().elem0) + o.blocks.back().n_elem;
     o.idx.assign(n, -1);
     o.src.assign(n, -1);
@@ -222,8 +229,8 @@ void fill_resident(const HostCsr& csr, HostResident& o) {
                 if (m.slot >= 0) {
                     const ResLong& l = o.longs[B.long0 + ln];
                     const int32_t row = B.row0 + l.row;
-                    k0 = rp[row] + (m.slot - l.slot0) * kResPiece;
-                    k1 = std::min(k0 + kResPiece, rp[row + 1]);
+                    k0 = rp[row] + (m.slot - l.slot0) * piece;
+                    k1 = std::min(k0 + piece, rp[row + 1]);
                 } else {
                     k0 = rp[B.row0 + ln];
                     k1 = rp[B.row0 + ln + 1];

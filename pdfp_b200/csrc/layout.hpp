@@ -233,11 +233,11 @@ void interleave_tiles(const HostTiling& in, int nseg, HostTiling& out);
 // block b owns the packed rows [row0, row1), cut into SLICES of 32 lanes.  A slice
 // holds 32 >> lg rows with 2^lg lanes each; lane l's entries are idx[off + u * 32 + l],
 // u = 0 .. depth-1 (index -1: no entry), its row is lane_row[slice * 32 + l] (relative
-// to row0, -1: none).  A row of more than kResPiece nonzeros takes several slices of
+// to row0, -1: none).  A row of more than 32 * lane_nnz nonzeros takes several slices of
 // one row each (slot >= 0: the slice's partial-sum slot; lane_row then holds the row's
 // ResLong in the block's list), whose sums are added in slot order.
 constexpr int kResLaneNnz = 32;  // nonzeros per lane that set a row's lanes (a power of two up to 32)
-constexpr int kResPiece = 1024;  // nonzeros per slice of a long row (32 per lane)
+constexpr int kCluLaneNnz = 16;  // the same for a small member's cluster
 
 struct alignas(16) ResSlice {
     int32_t off;    // first entry, relative to the block's entries
@@ -260,14 +260,16 @@ struct HostResident {
     std::vector<int32_t> lane_row;  // 32 per slice
     std::vector<int32_t> idx, src;  // per entry: gathered index and CSR position (-1: none)
 };
-// Deals the rows to n_blocks contiguous ranges of about equal nonzeros + 4 per row.
-// A row's lanes, and with them the order in which its terms are added, depend on its
-// length alone, never on its block.
-// deal_resident makes the blocks, slices and rows (which tell what a block's shared
-// memory must hold), fill_resident then the entries.
-void deal_resident(const HostCsr& csr, const std::vector<int32_t>& inst_row_off, int n_blocks,
-                   HostResident& out);
-void fill_resident(const HostCsr& csr, HostResident& out);
+// Deals the rows to contiguous ranges of about equal nonzeros + 4 per row (per_member: 64
+// per row, since a warp there has the same few rows whatever their length): n_blocks of
+// them, or n_blocks of each instance in turn (per_member).  A row's lanes (about lane_nnz
+// nonzeros each), and with them the order in which its terms are added, depend on its
+// length alone, never on its block.  deal_resident makes the blocks, slices and rows
+// (which tell what a block's shared memory must hold), fill_resident then the entries.
+// Slice depths are rounded up to a multiple of depth_unit.
+void deal_resident(const HostCsr& csr, const std::vector<int32_t>& inst_row_off, int n_blocks, int lane_nnz,
+                   int depth_unit, bool per_member, HostResident& out);
+void fill_resident(const HostCsr& csr, int lane_nnz, HostResident& out);
 // Dynamic shared memory a block needs for its share of both sides, with `esize`-byte
 // reals, ncv / nrv vectors kept per column / row and par_bytes of parameters per
 // instance; `shared`: one set of products serves both sides in turn.  The kernel carves
@@ -305,6 +307,35 @@ PDFP_HD inline ResSmem res_smem(const ResBlock& t, const ResBlock& a, int esize,
     s.long_a = take(uint64_t(16) * a.n_long);
     s.arr_t = take(uint64_t(4) * t.n_long);
     s.arr_a = take(uint64_t(4) * a.n_long);
+    s.total = off;
+    return s;
+}
+
+// Dynamic shared memory of one block of a small member's cluster (cluster_windows.cuh):
+// its slices' entries, the member's x_bar and z (with one entry more, the zero that empty
+// lanes gather) and the evaluation's partial sums.
+constexpr int kCluDepthUnit = 4;
+constexpr int kCluEvalRows = 32;  // rows per partial sum of an evaluation
+struct CluSmem {
+    uint32_t xs, zs, part_c, part_r, val_t, val_a, idx_t, idx_a, total;
+};
+PDFP_HD inline CluSmem clu_smem(const ResBlock& t, const ResBlock& a, int esize, int32_t n, int32_t m) {
+    CluSmem s;
+    uint32_t off = 0;
+    auto take = [&](uint64_t bytes) {
+        const uint32_t at = off;
+        off += static_cast<uint32_t>((bytes + 15) & ~uint64_t(15));
+        return at;
+    };
+    // first what other blocks write: at the same place in every block of the cluster
+    s.xs = take(uint64_t(esize) * (n + 1));
+    s.zs = take(uint64_t(esize) * (m + 1));
+    s.part_c = take(uint64_t(64) * ((n + kCluEvalRows - 1) / kCluEvalRows));
+    s.part_r = take(uint64_t(32) * ((m + kCluEvalRows - 1) / kCluEvalRows));
+    s.val_t = take(uint64_t(esize) * t.n_elem);
+    s.val_a = take(uint64_t(esize) * a.n_elem);
+    s.idx_t = take(uint64_t(4) * t.n_elem);
+    s.idx_a = take(uint64_t(4) * a.n_elem);
     s.total = off;
     return s;
 }

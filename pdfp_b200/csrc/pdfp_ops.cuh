@@ -62,24 +62,33 @@ __device__ __forceinline__ StepParams<T> step_params(const InstState& st, int32_
 }
 
 // primal_step! and dual_y_step! of one column (src/pdfp.jl:119-143): pv = {x, x0, y, y0,
-// l, u, x~, w} (w < 0 marks a column outside I), sum = (A'z)_j.
+// l, u, x~, w} (w < 0 marks a column outside I), sum = (A'z)_j.  primal_x gives what the
+// rows wait for, primal_rest the column's own new iterates.
 template <typename T>
-struct PrimalCell {
-    T cx, rx, cy;          // the new iterates and x_bar
-    T px, t, py, ry;       // x_hat, its unclamped argument, y_hat, reflected y (major steps)
+struct PrimalX {
+    T t, px, rx;  // the unclamped argument of x_hat, x_hat, x_bar
 };
 template <typename T>
-__device__ __forceinline__ PrimalCell<T> primal_cell(const StepParams<T>& p, const T (&pv)[8], T sum) {
-    const T cx = pv[0], ix = pv[1], cy = pv[2], iy = pv[3];
-    const T lb = pv[4], ub = pv[5], xt = pv[6], w = pv[7];
-    PrimalCell<T> o;
+struct PrimalRest {
+    T cx, cy, py, ry;  // the new iterates, y_hat and its reflection
+};
+template <typename T>
+__device__ __forceinline__ PrimalX<T> primal_x(const StepParams<T>& p, const T (&pv)[8], T sum) {
+    const T cx = pv[0], cy = pv[2], lb = pv[4], ub = pv[5];
+    PrimalX<T> o;
     // primal_step!  (src/pdfp.jl:124-129)
     o.t = sub_rn(cx, mul_rn(p.tau, sub_rn(sum, cy)));
     o.px = jl_clamp(o.t, lb, ub);
     o.rx = sub_rn(mul_rn(T(2), o.px), cx);
-    o.cx = halpern(p.weight, p.omega, p.omw, p.omwt, o.rx, cx, ix);
+    return o;
+}
+template <typename T>
+__device__ __forceinline__ PrimalRest<T> primal_rest(const StepParams<T>& p, const T (&pv)[8], T rx) {
+    const T cx = pv[0], ix = pv[1], cy = pv[2], iy = pv[3], xt = pv[6], w = pv[7];
+    PrimalRest<T> o;
+    o.cx = halpern(p.weight, p.omega, p.omw, p.omwt, rx, cx, ix);
     // dual_y_step!  (src/pdfp.jl:138-141); w < 0 marks j outside I
-    o.py = w >= T(0) ? jl_clamp(add_rn(cy, mul_rn(p.sigma, sub_rn(xt, o.rx))), -w, w) : T(0);
+    o.py = w >= T(0) ? jl_clamp(add_rn(cy, mul_rn(p.sigma, sub_rn(xt, rx))), -w, w) : T(0);
     o.ry = sub_rn(mul_rn(T(2), o.py), cy);
     o.cy = halpern(p.weight, p.omega, p.omw, p.omwt, o.ry, cy, iy);
     return o;
@@ -156,13 +165,14 @@ struct PrimalOp {
     }
     // The epilogue on column j's inputs pv (staged() order) and its sum s = (A'z)_j.
     __device__ void row_vals(int32_t j, const TileP& p, const T (&pv)[NVEC], const T (&s)[1]) const {
-        const PrimalCell<T> o = primal_cell(p, pv, s[0]);
+        const PrimalX<T> x = primal_x(p, pv, s[0]);
+        const PrimalRest<T> o = primal_rest(p, pv, x.rx);
         v.cx[j] = o.cx;
-        v.rx[j] = o.rx;
+        v.rx[j] = x.rx;
         v.cy[j] = o.cy;
         if (MAJOR) {
-            v.px[j] = o.px;
-            v.ds[j] = sub_rn(o.px, o.t) / p.tau;
+            v.px[j] = x.px;
+            v.ds[j] = sub_rn(x.px, x.t) / p.tau;
             v.py[j] = o.py;
             v.ry[j] = o.ry;
         }

@@ -18,6 +18,7 @@
 #include "device.hpp"
 #include "kernels.cuh"
 #include "pdlp_ops.cuh"
+#include "cluster_windows.cuh"
 #include "resident_steps.cuh"
 #include "tiny_steps.cuh"
 #include "power.cuh"
@@ -237,6 +238,36 @@ struct LpRestartCopy {
             v.cy[r] = y;
         }
     }
+};
+
+// A small LP's whole windows in one launch (cluster_windows.cuh), without the cuPDLPx ray
+// passes.
+template <typename TT>
+struct LpCluster : LpResident<TT> {
+    using T = TT;
+    using B = LpResident<TT>;
+    using EvalCol = LpEvalColOp<T, kCluThreads>;
+    using EvalRow = LpEvalRowOp<T, kCluThreads>;
+    LpData d;
+    InstState* stw;
+    InstFlags* fl;
+    __device__ EvalCol eval_col(int32_t which) const { return EvalCol{B::v, d, B::st, which, B::mode, B::errp}; }
+    __device__ EvalRow eval_row(int32_t which) const { return EvalRow{B::v, d, B::st, which, B::mode, B::errp}; }
+    __device__ void finalize(int p, const double* a, int32_t which) const {
+        LpController{nullptr, nullptr, nullptr, nullptr, stw, fl, which == EVAL_FULL ? 1 : 0, 0}.finalize(p, a);
+    }
+    __device__ bool polish(int p) const { return fl[p].polish_request != 0; }
+    __device__ void col_restart(int32_t j, T* v) const {
+        const T x = B::v.px[j];
+        B::v.ix[j] = x;
+        v[0] = v[1] = x;
+    }
+    __device__ void row_restart(int32_t i, T* v) const {
+        const T y = B::v.py[i];
+        B::v.iy[i] = y;
+        v[0] = v[1] = y;
+    }
+    __device__ const T* row_pdhg() const { return B::v.py; }
 };
 
 // ---- a small LP's whole solve in one launch ---------------------------------------------
@@ -602,6 +633,7 @@ class LpSolver {
     const DeviceMatrix::Tiling& tiling_a() const {
         return (std::is_same<T, double>::value && f32_) ? it64_a_ : it_a_;
     }
+    ClusterForm clu32_, clu64_;   // a small LP's whole windows, where it fits
     ResidentForm res32_, res64_;  // the window's steps with the LP on the chip, where it fits
     template <typename T>
     ResidentForm& resident() {
@@ -684,6 +716,18 @@ template <typename T>
 void LpSolver::launch_tiny_solve() {
     LpVecs<T>* vp = nullptr;
     if constexpr (std::is_same<T, float>::value) vp = &v32_; else vp = &v64_;
+    ClusterForm& cf = std::is_same<T, float>::value ? clu32_ : clu64_;
+    if (!cupdlpx_) cf.template prepare<LpCluster<T>>(M_, ar_, max_smem_, stream_);
+    if (cf.ready()) {
+        LpCluster<T> prob;
+        static_cast<LpResident<T>&>(prob) =
+            LpResident<T>{*vp, st_, std::is_same<T, float>::value ? MODE_FP32 : MODE_FP64, err_};
+        prob.d = d_;
+        prob.stw = st_;
+        prob.fl = flags_;
+        cf.launch(prob, M_, nullptr, stream_);
+        return;
+    }
     const int32_t rowsum_len = 2 * std::max(std::max(n_, m_), 1);
     const size_t base = sizeof(double) * static_cast<size_t>(rowsum_len);
     // the staged form when the LP's copy fits next to the row sums (PDFP_TINY_STAGE=0: in place)

@@ -45,17 +45,16 @@ __device__ __forceinline__ void atomic_max_nonneg(unsigned long long* slot, doub
 // primal_step! of one column (src/pdlp.jl:115-132; tau is the primal step): pv = {x, x0,
 // c, l, u}, sum = (A'y)_j.
 template <typename T>
-struct LpPrimalCell {
-    T cx, rx, px, t;  // the new iterate, x_bar, x_hat and its unclamped argument
+struct LpPrimalX {
+    T rx, px, t;  // x_bar, x_hat and its unclamped argument
 };
 template <typename T>
-__device__ __forceinline__ LpPrimalCell<T> lp_primal_cell(const StepParams<T>& p, const T (&pv)[5], T sum) {
-    const T cx = pv[0], ix = pv[1], c = pv[2], lb = pv[3], ub = pv[4];
-    LpPrimalCell<T> o;
+__device__ __forceinline__ LpPrimalX<T> lp_primal_x(const StepParams<T>& p, const T (&pv)[5], T sum) {
+    const T cx = pv[0], c = pv[2], lb = pv[3], ub = pv[4];
+    LpPrimalX<T> o;
     o.t = sub_rn(cx, mul_rn(p.tau, sub_rn(c, sum)));
     o.px = jl_clamp(o.t, lb, ub);
     o.rx = sub_rn(mul_rn(T(2), o.px), cx);
-    o.cx = halpern(p.weight, p.omega, p.omw, p.omwt, o.rx, cx, ix);
     return o;
 }
 
@@ -101,11 +100,11 @@ struct LpPrimalOp {
     __device__ void row(int32_t j, int32_t rr, int, const TileP& p, const T* const* sv,
                         const T (&s)[1], double*) const {
         const T pv[5] = {sv[0][rr], sv[1][rr], sv[2][rr], sv[3][rr], sv[4][rr]};
-        const LpPrimalCell<T> o = lp_primal_cell(p, pv, s[0]);
+        const LpPrimalX<T> o = lp_primal_x(p, pv, s[0]);
         if (MAJOR) v.ds[j] = sub_rn(o.px, o.t) / p.tau;
         v.px[j] = o.px;
         v.rx[j] = o.rx;
-        v.cx[j] = o.cx;
+        v.cx[j] = halpern(p.weight, p.omega, p.omw, p.omwt, o.rx, pv[0], pv[1]);
     }
     __device__ void write_partials(int32_t, const double*) const {}
 };
@@ -162,17 +161,19 @@ struct LpResident {
         T* const s[NRV] = {v.cy, v.iy, v.clb, v.cub};
         return s[q];
     }
+    using X = LpPrimalX<T>;
+    __device__ __forceinline__ X col_x(const StepParams<T>& p, const T (&in)[NCV], T sum) const {
+        return lp_primal_x(p, in, sum);
+    }
     template <bool MAJOR>
-    __device__ __forceinline__ T col(const StepParams<T>& p, int32_t j, const T (&in)[NCV], T* pv, int,
-                                     T sum) const {
-        const LpPrimalCell<T> o = lp_primal_cell(p, in, sum);
-        pv[0] = o.cx;
+    __device__ __forceinline__ void col_rest(const StepParams<T>& p, int32_t j, const T (&in)[NCV], const X& x,
+                                             T* pv, int) const {
+        pv[0] = halpern(p.weight, p.omega, p.omw, p.omwt, x.rx, in[0], in[1]);
         if (MAJOR) {
-            v.ds[j] = sub_rn(o.px, o.t) / p.tau;
-            v.px[j] = o.px;
-            v.rx[j] = o.rx;
+            v.ds[j] = sub_rn(x.px, x.t) / p.tau;
+            v.px[j] = x.px;
+            v.rx[j] = x.rx;
         }
-        return o.rx;
     }
     template <bool MAJOR>
     __device__ __forceinline__ T row(const StepParams<T>& p, bool, int32_t i, const T (&in)[NRV], T* pv, int,

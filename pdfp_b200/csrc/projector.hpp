@@ -15,6 +15,7 @@
 namespace pdfp {
 
 struct ResidentForm;  // resident_steps.cuh
+struct ClusterForm;   // cluster_windows.cuh
 
 // One projection problem in the caller's numbering (scaled data).
 struct ProblemData {
@@ -148,12 +149,13 @@ class Projector {
     void launch_resident_steps(int i0, int i1);
     template <typename T>
     ResidentForm& ensure_resident();
+    template <typename T>
+    ClusterForm& ensure_cluster();
+    template <typename T>
+    void launch_cluster();
     cudaGraphExec_t window_graph(int freq, bool with32, bool with64);
     void prepare_window();
     void run_window(int freq, bool with32, bool with64);
-    bool window_ready_ = false;  // the whole-window kernels' launch shape is set
-    size_t tiny_smem32_ = 0, tiny_smem64_ = 0;      // their dynamic shared memory
-    bool tiny_staged32_ = false, tiny_staged64_ = false;  // members copied into shared memory
 
     int precision_;
     int K_ = 0;
@@ -215,6 +217,7 @@ class Projector {
     // each precision's form once a window needed it.
     bool resident_ = false;
     std::shared_ptr<ResidentForm> res32_, res64_;
+    std::shared_ptr<ClusterForm> clu32_, clu64_;  // small members: whole windows in one launch
     bool vecwin_ = false;  // FP32 minor steps of a window in one cooperative vec launch
     int vecwin_grid_ = 0;  // its blocks (all resident)
     void launch_vec_window(int i0, int i1);

@@ -97,21 +97,25 @@ struct PdfpResident {
         T* const s[NRV] = {v.cz, v.iz, v.b};
         return s[q];
     }
-    // column j with its vectors, read as `in`, at pv[q * n] in shared memory; returns x_bar_j
+    // column j with its vectors, read as `in`, at pv[q * n]: first x_bar_j (.rx), for which
+    // others wait, then its own iterates
+    using X = PrimalX<T>;
+    __device__ __forceinline__ X col_x(const StepParams<T>& p, const T (&in)[NCV], T sum) const {
+        return primal_x(p, in, sum);
+    }
     template <bool MAJOR>
-    __device__ __forceinline__ T col(const StepParams<T>& p, int32_t j, const T (&in)[NCV], T* pv, int n,
-                                     T sum) const {
-        const PrimalCell<T> o = primal_cell(p, in, sum);
+    __device__ __forceinline__ void col_rest(const StepParams<T>& p, int32_t j, const T (&in)[NCV], const X& x,
+                                             T* pv, int n) const {
+        const PrimalRest<T> o = primal_rest(p, in, x.rx);
         pv[0] = o.cx;
         pv[2 * n] = o.cy;
         if (MAJOR) {
-            v.rx[j] = o.rx;
-            v.px[j] = o.px;
-            v.ds[j] = sub_rn(o.px, o.t) / p.tau;
+            v.rx[j] = x.rx;
+            v.px[j] = x.px;
+            v.ds[j] = sub_rn(x.px, x.t) / p.tau;
             v.py[j] = o.py;
             v.ry[j] = o.ry;
         }
-        return o.rx;
     }
     // row i likewise; returns z_i
     template <bool MAJOR>
@@ -322,16 +326,16 @@ __device__ __forceinline__ void res_pass(const P& prob, unsigned char* sm, const
             }
             if (r >= 0) {
                 const int32_t i = s.row0 + r;
-                T v;
                 if (is_row) {
                     T in3[P::NRV];
 #pragma unroll
                     for (int e = 0; e < P::NRV; ++e) in3[e] = in[e];
-                    v = prob.template row<MAJOR>(p, i < pr.eq_end, i, in3, pv, s.rows, acc);
+                    res_put(s.out + i, prob.template row<MAJOR>(p, i < pr.eq_end, i, in3, pv, s.rows, acc), k + 1);
                 } else {
-                    v = prob.template col<MAJOR>(p, i, in, pv, s.rows, acc);
+                    const typename P::X x = prob.col_x(p, in, acc);
+                    res_put(s.out + i, x.rx, k);
+                    prob.template col_rest<MAJOR>(p, i, in, x, pv, s.rows);
                 }
-                res_put(s.out + i, v, is_row ? k + 1 : k);
             }
             __syncwarp();
         }

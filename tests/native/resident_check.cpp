@@ -12,11 +12,15 @@ using namespace pdfp;
 
 // The order in which a row's nonzeros are added, as one number per nonzero: its place
 // in the slice (depth and lane relative to the row's first lane, piece).
-static int check_side(const HostCsr& csr, const std::vector<int32_t>& off, int n_blocks,
-                      HostResident& h) {
-    deal_resident(csr, off, n_blocks, h);
-    fill_resident(csr, h);
-    if (static_cast<int>(h.blocks.size()) != n_blocks) return 1;
+static int check_side(const HostCsr& csr, const std::vector<int32_t>& off, int n_blocks, int lane_nnz,
+                      int unit, bool per_member, HostResident& h) {
+    const int kResLaneNnz = lane_nnz, kResPiece = 32 * lane_nnz;
+    deal_resident(csr, off, n_blocks, lane_nnz, unit, per_member, h);
+    fill_resident(csr, lane_nnz, h);
+    const int K = static_cast<int>(off.size()) - 1;
+    if (static_cast<int>(h.blocks.size()) != (per_member ? K : 1) * n_blocks) return 1;
+    for (size_t b = 0; per_member && b < h.blocks.size(); ++b)  // a member's blocks hold its rows
+        if (h.blocks[b].row0 < off[b / n_blocks] || h.blocks[b].row1 > off[b / n_blocks + 1]) return 24;
     if (h.lane_row.size() != 32 * h.slices.size() || h.idx.size() != h.src.size()) return 2;
     std::vector<int> rows_done(csr.rows, 0), nz_done(csr.ci.size(), 0);
     int32_t next_row = 0, next_slice = 0, next_elem = 0, next_long = 0;
@@ -45,7 +49,7 @@ static int check_side(const HostCsr& csr, const std::vector<int32_t>& off, int n
         for (int32_t q = 0; q < b.n_slices; ++q) {
             const ResSlice& m = h.slices[b.slice0 + q];
             const int lg = m.shape & 7, depth = m.shape >> 3, G = 1 << lg;
-            if (lg > 5 || depth < 0 || m.off < 0 || m.off + 32 * depth > b.n_elem) return 10;
+            if (lg > 5 || depth < 0 || depth % unit || m.off < 0 || m.off + 32 * depth > b.n_elem) return 10;
             if (m.inst < 0 || m.inst >= b.n_inst) return 11;
             if (q > 0 && depth > (h.slices[b.slice0 + q - 1].shape >> 3)) return 12;
             for (int lane = 0; lane < 32; ++lane) {
@@ -99,8 +103,20 @@ extern "C" int resident_check(int K, const int32_t* ms, const int32_t* ns, const
         HostLayout L;
         if (!build_layout(probs, permute != 0, L).empty()) return 100;
         HostResident t, a;
-        if (int rc = check_side(L.At, L.col_off, n_blocks, t)) return 200 + rc;
-        if (int rc = check_side(L.A, L.row_off, n_blocks, a)) return 300 + rc;
+        for (int c = 1; c <= 8; ++c) {  // small members' clusters
+            if (int rc = check_side(L.At, L.col_off, c, kCluLaneNnz, kCluDepthUnit, true, t)) return 500 + rc;
+            if (int rc = check_side(L.A, L.row_off, c, kCluLaneNnz, kCluDepthUnit, true, a)) return 600 + rc;
+            for (size_t b = 0; b < t.blocks.size(); ++b) {
+                const CluSmem s = clu_smem(t.blocks[b], a.blocks[b], 8, ns[b / c], ms[b / c]);
+                if (s.total % 16 || s.idx_a > s.total) return 700;
+                // what other blocks write lies at the same place in all of a member's blocks
+                const size_t f = b / c * c;
+                const CluSmem s0 = clu_smem(t.blocks[f], a.blocks[f], 8, ns[b / c], ms[b / c]);
+                if (s.xs != s0.xs || s.zs != s0.zs || s.part_c != s0.part_c || s.part_r != s0.part_r) return 701;
+            }
+        }
+        if (int rc = check_side(L.At, L.col_off, n_blocks, kResLaneNnz, 1, false, t)) return 200 + rc;
+        if (int rc = check_side(L.A, L.row_off, n_blocks, kResLaneNnz, 1, false, a)) return 300 + rc;
         stats[0] = stats[1] = 0;
         for (int b = 0; b < n_blocks; ++b) {
             const ResSmem s = res_smem(t.blocks[b], a.blocks[b], 8, 8, 3, 48, (b & 1) != 0);

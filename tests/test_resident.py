@@ -152,3 +152,76 @@ def test_batch_members_equal_single_handles(oracle, monkeypatch, precision):
         assert s.total_count == b.results[p]["total_count"] == 200 * (1 + p % 3)
         x, y = s.pdhg_x, b.get(p, "pdhg_x")
         assert np.linalg.norm(x - y) <= tol * max(1.0, np.linalg.norm(x)), p
+
+
+# ---- small members: whole windows in a thread-block cluster (cluster_windows.cuh) -------
+
+
+def _small_models():
+    """One, two and several blocks per member; sizes at the edges of a warp's 32 rows; dense
+    rows shared by several lanes; rows and columns without entries."""
+    out = [synthetic.covering_p0201_like(1), synthetic.markshare_like(2)]
+    for seed, m, n, mean in ((3, 31, 33, 4.0), (4, 64, 97, 3.0), (5, 211, 305, 7.5), (6, 601, 1503, 25.0)):
+        out.append(synthetic.general_integer(seed, m=m, n=n, m_eq=m // 4, mean_row=mean)[0])
+    return out
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_small_members_match_oracle_and_their_batch(oracle, precision):
+    """One and three windows of each member: against the oracle (the bounds of the resident
+    steps' test), and in one batch handle, whose cluster size is another: bit for bit."""
+    from pdfp_b200 import gpu
+    tol = 1e-10 if precision == "fp64" else 2e-4
+    probs, targets, singles = [], [], []
+    for k, m in enumerate(_small_models()):
+        sc, is_eq, is_int, w = oracle.projector_inputs(m)
+        probs.append((sc.A, sc.con_ub, is_eq, is_int, sc.var_lb, sc.var_ub, w))
+        rng = np.random.default_rng(30 + k)
+        xt = np.zeros(len(m.c))
+        xt[m.int_idx] = np.round(m.l[m.int_idx] + rng.random(len(m.int_idx)) * (m.u - m.l)[m.int_idx])
+        targets.append(xt / sc.D_c)
+    for windows in (1, 3):
+        prm = SolverParameters(eps_optimal_relative=1e-9, eps_feasible_relative=1e-9,
+                               iteration_limit=200 * windows)
+        batch = gpu.PDFPBatch(probs, precision=precision)
+        for p, xt in enumerate(targets):
+            batch.set_target(p, xt)
+        batch.solve(prm, 1.0)
+        for p, pr in enumerate(probs):
+            s, o = gpu.PDFPState(*pr, precision=precision), oracle.OracleSolvers.PDFPState(*pr)
+            form = gpu.C.c_int32()
+            gpu.L.check(gpu.L.lib().pdfp_get_window_form(s._h, gpu.C.byref(form)))
+            assert form.value == 3
+            for h in (s, o):
+                h.set_target(targets[p])
+                h.solve(prm, 1.0)
+            assert s.total_count == batch.results[p]["total_count"]
+            for name in ("pdhg_x", "pdhg_y", "pdhg_z", "current_x", "current_y", "current_z", "dual_slack"):
+                a, b = s.get(name), o.get(name)
+                if s.total_count == 200 * windows:
+                    assert np.linalg.norm(a - b) <= tol * max(1.0, np.linalg.norm(b)), (p, windows, name)
+                assert np.array_equal(a, batch.get(p, name)), (p, windows, name)
+
+
+@pytest.mark.gpu
+def test_a_row_too_long_for_a_cluster_takes_the_resident_steps(oracle):
+    """A row of more than 512 nonzeros, and a member of as many rows as a cluster has no
+    warps for: the handle runs its windows resident on the chip instead."""
+    from pdfp_b200 import gpu
+    rng = np.random.default_rng(8)
+    A = sp.random(40, 700, density=0.01, random_state=rng, format="lil")
+    A[7, :] = rng.uniform(-1.0, 1.0, size=700)
+    A = sp.csr_matrix(A)
+    for mat in (A, sp.csr_matrix(sp.random(1900, 2100, density=0.004, random_state=rng))):
+        m, n = mat.shape
+        b = mat @ rng.random(n) + 0.5
+        pr = (mat, b, np.zeros(m, np.uint8), np.ones(n, np.uint8), np.zeros(n), np.ones(n), np.ones(n))
+        s, o = gpu.PDFPState(*pr), oracle.OracleSolvers.PDFPState(*pr)
+        prm = SolverParameters(eps_optimal_relative=1e-9, eps_feasible_relative=1e-9, iteration_limit=400)
+        xt = np.round(rng.random(n))
+        for h in (s, o):
+            h.set_target(xt)
+            h.solve(prm, 1.0)
+        assert s.total_count == o.total_count
+        assert np.linalg.norm(s.pdhg_x - o.pdhg_x) <= 1e-10 * max(1.0, np.linalg.norm(o.pdhg_x))
