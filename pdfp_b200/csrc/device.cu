@@ -260,18 +260,14 @@ bool DeviceMatrix::make_resident(DeviceArena& ar, int n_blocks, int esize, int n
                                  int par_bytes, uint32_t max_smem, Resident& r) const {
     r = Resident();
     // entries and vectors alone, spread evenly: no need to lay out what cannot fit
-    const double least = 2.0 * L.NNZ * (4 + esize) + 1.0 * L.NNZ * esize +
+    const double least = 2.0 * L.NNZ * (4 + 2 * esize) +
                          static_cast<double>(esize * ncv + 4) * L.N + static_cast<double>(esize * nrv + 4) * L.M;
     if (n_blocks <= 0 || least > static_cast<double>(n_blocks) * max_smem) return false;
     HostResident ht, ha;
     deal_resident(L.At, L.col_off, n_blocks, kResLaneNnz, 1, false, ht);
     deal_resident(L.A, L.row_off, n_blocks, kResLaneNnz, 1, false, ha);
-    for (int shared = 0; shared < 2 && (shared == 0 || r.smem > max_smem); ++shared) {
-        r.smem = 0;
-        r.shared = shared != 0;
-        for (int b = 0; b < n_blocks; ++b)
-            r.smem = std::max(r.smem, res_smem(ht.blocks[b], ha.blocks[b], esize, ncv, nrv, par_bytes, r.shared).total);
-    }
+    for (int b = 0; b < n_blocks; ++b)
+        r.smem = std::max(r.smem, res_smem(ht.blocks[b], ha.blocks[b], esize, ncv, nrv, par_bytes).total);
     if (r.smem > max_smem) return false;
     upload_resident(ar, ht, ha, kResLaneNnz, r);
     return true;

@@ -184,8 +184,7 @@ class DeviceMatrix {
         const int32_t *src_t = nullptr, *src_a = nullptr;  // CSR position of each entry (-1: none)
         int64_t n_t = 0, n_a = 0;                          // entries
         int n_blocks = 0;
-        bool shared = false;  // one set of products serves both sides
-        uint32_t smem = 0;    // dynamic shared memory of the largest block
+        uint32_t smem = 0;  // dynamic shared memory of the largest block
     };
     bool make_resident(DeviceArena& ar, int n_blocks, int esize, int ncv, int nrv, int par_bytes,
                        uint32_t max_smem, Resident& out) const;

@@ -272,14 +272,13 @@ void deal_resident(const HostCsr& csr, const std::vector<int32_t>& inst_row_off,
 void fill_resident(const HostCsr& csr, int lane_nnz, HostResident& out);
 // Dynamic shared memory a block needs for its share of both sides, with `esize`-byte
 // reals, ncv / nrv vectors kept per column / row and par_bytes of parameters per
-// instance; `shared`: one set of products serves both sides in turn.  The kernel carves
-// its memory with the same function.
+// instance.  The kernel carves its memory with the same function.
 struct ResSmem {
     uint32_t col, row, val_t, val_a, prod_t, prod_a, par_t, par_a, slots_t, slots_a, idx_t, idx_a, lane_t, lane_a,
         slice_t, slice_a, long_t, long_a, arr_t, arr_a, total;
 };
 PDFP_HD inline ResSmem res_smem(const ResBlock& t, const ResBlock& a, int esize, int ncv, int nrv,
-                                int par_bytes, bool shared) {
+                                int par_bytes) {
     ResSmem s;
     uint32_t off = 0;
     auto take = [&](uint64_t bytes) {
@@ -291,8 +290,8 @@ PDFP_HD inline ResSmem res_smem(const ResBlock& t, const ResBlock& a, int esize,
     s.row = take(uint64_t(esize) * nrv * (a.row1 - a.row0));
     s.val_t = take(uint64_t(esize) * t.n_elem);
     s.val_a = take(uint64_t(esize) * a.n_elem);
-    s.prod_t = take(uint64_t(esize) * (shared && a.n_elem > t.n_elem ? a.n_elem : t.n_elem));
-    s.prod_a = shared ? s.prod_t : take(uint64_t(esize) * a.n_elem);
+    s.prod_t = take(uint64_t(esize) * t.n_elem);
+    s.prod_a = take(uint64_t(esize) * a.n_elem);
     s.par_t = take(uint64_t(par_bytes) * t.n_inst);
     s.par_a = take(uint64_t(par_bytes) * a.n_inst);
     s.slots_t = take(uint64_t(8) * t.n_slots);

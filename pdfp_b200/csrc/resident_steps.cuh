@@ -27,6 +27,7 @@
 // take every 2^lg-th term, then an xor tree; pieces of a long row in order), so a batch
 // member takes the steps of its own handle bit for bit.
 #pragma once
+#include <algorithm>
 #include <type_traits>
 
 #include "common.cuh"
@@ -222,14 +223,14 @@ __device__ __forceinline__ T res_sum(const T* pp, int depth) {
 //     products in order and runs the epilogue: as many rows per FP64 instruction as
 //     lanes.  The other warps are already waiting for the next pass's entries.
 // The products of the two sides have their own memory, so the next pass may form its
-// products while this one's are summed (`shared`: they do not fit, and it waits).
+// products while this one's are summed.
 // Both sides run through the same code, and what is rare (major steps, long rows, the
 // wait's limit) stays out of it: a step is one pass through a few hundred instructions
 // by warps that have just been idle, so instructions that miss the small instruction
 // cache cost more than the arithmetic.
 template <class P, bool MAJOR>
 __device__ __forceinline__ void res_pass(const P& prob, unsigned char* sm, const ResSide<typename P::T>& s,
-                                         bool is_row, int32_t k, bool shared, unsigned* dead, bool& off) {
+                                         bool is_row, int32_t k, unsigned* dead, bool& off) {
     using T = typename P::T;
     constexpr int U = 4;  // gathers in flight per thread: 2 and 8 measured slower (1.92 and 2.29 ms for 1.87)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -268,7 +269,6 @@ __device__ __forceinline__ void res_pass(const P& prob, unsigned char* sm, const
         }
     }
     __syncwarp();
-    if (shared) __syncthreads();  // the other side's sums are done
 #pragma unroll 1
     for (int32_t e0 = threadIdx.x; e0 < s.n_elem; e0 += U * kResThreads) {
         int32_t c[U], t[U];
@@ -350,8 +350,7 @@ __device__ __forceinline__ void res_pass(const P& prob, unsigned char* sm, const
 template <class P>
 __global__ void __launch_bounds__(kResThreads, 1)
     resident_steps_kernel(const P prob, const ResDev dt, const ResDev da, ResWord<typename P::T>* wx,
-                          ResWord<typename P::T>* wz, unsigned* dead, int K, int32_t shared, int32_t i0,
-                          int32_t i1) {
+                          ResWord<typename P::T>* wz, unsigned* dead, int K, int32_t i0, int32_t i1) {
     using T = typename P::T;
     extern __shared__ __align__(16) unsigned char sm[];
     __shared__ ResSide<T> sides[2];  // 0: columns, 1: rows
@@ -360,7 +359,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
     if (!__syncthreads_or(any)) return;  // the same answer in every block
     {
         const ResBlock bt = dt.blocks[blockIdx.x], ba = da.blocks[blockIdx.x];
-        const ResSmem o = res_smem(bt, ba, sizeof(T), P::NCV, P::NRV, sizeof(ResPar<T>), shared != 0);
+        const ResSmem o = res_smem(bt, ba, sizeof(T), P::NCV, P::NRV, sizeof(ResPar<T>));
         if (threadIdx.x == 0) {
             sides[0] = ResSide<T>{wz, wx, o.idx_t, o.val_t, o.prod_t, o.slice_t, o.lane_t, o.long_t, o.col,
                                   o.slots_t, o.arr_t, o.par_t, bt.n_slices, bt.n_elem, bt.row0,
@@ -433,10 +432,10 @@ __global__ void __launch_bounds__(kResThreads, 1)
     bool off = false;
 #pragma unroll 1
     for (int32_t h = 2 * i0; h < 2 * i1; ++h)
-        res_pass<P, false>(prob, sm, sides[h & 1], h & 1, h >> 1, shared != 0, dead, off);
+        res_pass<P, false>(prob, sm, sides[h & 1], h & 1, h >> 1, dead, off);
 #pragma unroll 1
     for (int h = 0; h < 2; ++h)
-        res_pass<P, true>(prob, sm, sides[h], h != 0, i1, shared != 0, dead, off);
+        res_pass<P, true>(prob, sm, sides[h], h != 0, i1, dead, off);
     __syncthreads();
 #pragma unroll 1
     for (int h = 0; h < 2; ++h) {
@@ -472,8 +471,13 @@ struct ResidentForm {
         if (!coop || M.L.NNZ == 0) return;
         const uint32_t cap = static_cast<uint32_t>(max_smem_block) - 1024;  // its static memory
         PDFP_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(cap)));
+        // Where it stops to pay: 400 iterations of general-integer models, resident against
+        // per-step launches, FP64 500k nonzeros (187 KB a block) 3.2 / 5.7 ms, 610k (about
+        // 226 KB) 5.1 / 7.5; mixed 900k (194 KB) 4.5 / 6.3, 970k (200 KB) 4.6 / 6.4, 1M
+        // (205 KB) 7.0 / 6.5: what shared memory takes, the gathers' misses lack in L1.
+        const uint32_t most = sizeof(T) == 4 ? std::min(cap, 200u * 1024u) : cap;
         DeviceMatrix::Resident f;
-        if (!M.make_resident(ar, num_sms, sizeof(T), P::NCV, P::NRV, sizeof(ResPar<T>), cap, f)) return;
+        if (!M.make_resident(ar, num_sms, sizeof(T), P::NCV, P::NRV, sizeof(ResPar<T>), most, f)) return;
         PDFP_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kResThreads, f.smem));
         if (per_sm < 1) return;
         M.fill_resident(ar, f, std::is_same<T, float>::value, stream);
@@ -503,7 +507,7 @@ struct ResidentForm {
         cfg.attrs = at;
         cfg.numAttrs = 1;
         PDFP_CK(cudaLaunchKernelEx(&cfg, resident_steps_kernel<P>, prob, r.t, r.a, wx, wz, dead, K,
-                                   r.shared ? 1 : 0, static_cast<int32_t>(i0), static_cast<int32_t>(i1)));
+                                   static_cast<int32_t>(i0), static_cast<int32_t>(i1)));
     }
 
   private:

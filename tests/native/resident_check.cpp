@@ -119,7 +119,7 @@ extern "C" int resident_check(int K, const int32_t* ms, const int32_t* ns, const
         if (int rc = check_side(L.A, L.row_off, n_blocks, kResLaneNnz, 1, false, a)) return 300 + rc;
         stats[0] = stats[1] = 0;
         for (int b = 0; b < n_blocks; ++b) {
-            const ResSmem s = res_smem(t.blocks[b], a.blocks[b], 8, 8, 3, 48, (b & 1) != 0);
+            const ResSmem s = res_smem(t.blocks[b], a.blocks[b], 8, 8, 3, 48);
             if (s.total % 16 || s.long_a > s.total) return 400;
             stats[0] = std::max<int64_t>(stats[0], s.total);
         }
