@@ -826,11 +826,10 @@ IterVecs<double>& Projector::vecs<double>() { return v64_; }
 template <typename T, bool MAJOR>
 void Projector::launch_primal(const StepSide& s, int k, bool overlap) {
     const int mode = std::is_same<T, float>::value ? MODE_FP32 : MODE_FP64;
-    if constexpr (std::is_same<T, float>::value)
-        if (s.engine == 2) {
-            launch_vec(s.vec, PrimalOp<T, MAJOR, kFlatThreads>{vecs<T>(), st_, k, mode, err_, s.gather_l2}, s.grid, stream_);
-            return;
-        }
+    if (s.engine == 2) {
+        launch_vec(s.vec, PrimalOp<T, MAJOR, kFlatThreads>{vecs<T>(), st_, k, mode, err_, s.gather_l2}, s.grid, stream_);
+        return;
+    }
     if (s.engine == 1)
         launch_flat(s.tiling.dev, PrimalOp<T, MAJOR, kFlatThreads>{vecs<T>(), st_, k, mode, err_, s.gather_l2}, s.qpt, s.grid, stream_);
     else if (s.nt == 256)
@@ -842,11 +841,11 @@ void Projector::launch_primal(const StepSide& s, int k, bool overlap) {
 template <typename T, bool MAJOR>
 void Projector::launch_dual(const StepSide& s, int k, bool overlap) {
     const int mode = std::is_same<T, float>::value ? MODE_FP32 : MODE_FP64;
+    if (s.engine == 2) {
+        launch_vec(s.vec, DualOp<T, MAJOR, kFlatThreads>{vecs<T>(), st_, M_.row_off, M_.n_eq, k, mode, err_, s.gather_l2}, s.grid, stream_);
+        return;
+    }
     if constexpr (std::is_same<T, float>::value) {
-        if (s.engine == 2) {
-            launch_vec(s.vec, DualOp<T, MAJOR, kFlatThreads>{vecs<T>(), st_, M_.row_off, M_.n_eq, k, mode, err_, s.gather_l2}, s.grid, stream_);
-            return;
-        }
         if (s.seg_nseg > 0) {  // the long rows first; the tile launch then follows no step launch
             launch_seg(s.segt.dev, s.segd, s.seg_nt, s.seg_bps,
                        DualOp<T, MAJOR, kFlatThreads>{vecs<T>(), st_, M_.row_off, M_.n_eq, k, mode, err_, s.gather_l2},
@@ -878,22 +877,27 @@ void Projector::prepare_side(StepSide& s, bool primal, bool f32) {
     const int e = f32 ? 4 : 8;
     if (s.engine != 0) s.seg_nseg = 0;  // segmented long rows: tile engine only
     if (s.engine == 2) {
-        if (!f32) throw Error(E_INVALID, "internal: the vec engine runs the FP32 steps only");
         // The A' side (short, even rows on the zipf-lp matrix: 68 us against 72 us a
         // launch) takes larger items while they leave at least two per warp of a full
         // grid; on the A side (Zipf-skewed rows) larger items measured slower.
         s.vec = M_.make_vec(ar_, primal, s.lane_nnz,
-                            primal ? int64_t(2) * num_sms_ * kVecMinBlocks * (kVecThreads / 32) : 0);
+                            primal ? int64_t(2) * num_sms_ * (f32 ? kVecMinBlocks : kVecMinBlocks64) * (kVecThreads / 32) : 0);
         s.stage_bytes = s.lane_nnz;
         s.nt = 32;
         s.half_red = false;
         if (s.gather_l2 == 2) s.gather_l2 = 1;
         // both the MAJOR and the minor kernel: the grid is the smaller of the two
-        const int g0 = primal ? vec_grid<PrimalOp<float, false, kFlatThreads>>(s.vec, num_sms_)
-                              : vec_grid<DualOp<float, false, kFlatThreads>>(s.vec, num_sms_);
-        const int g1 = primal ? vec_grid<PrimalOp<float, true, kFlatThreads>>(s.vec, num_sms_)
-                              : vec_grid<DualOp<float, true, kFlatThreads>>(s.vec, num_sms_);
-        s.grid = std::min(g0, g1);
+        auto grid = [&](auto minor, auto major) {
+            s.grid = std::min(vec_grid<decltype(minor)>(s.vec, num_sms_), vec_grid<decltype(major)>(s.vec, num_sms_));
+        };
+        if (primal && f32)
+            grid(PrimalOp<float, false, kFlatThreads>{}, PrimalOp<float, true, kFlatThreads>{});
+        else if (primal)
+            grid(PrimalOp<double, false, kFlatThreads>{}, PrimalOp<double, true, kFlatThreads>{});
+        else if (f32)
+            grid(DualOp<float, false, kFlatThreads>{}, DualOp<float, true, kFlatThreads>{});
+        else
+            grid(DualOp<double, false, kFlatThreads>{}, DualOp<double, true, kFlatThreads>{});
         return;
     }
     if (s.engine == 1) {
@@ -1000,10 +1004,13 @@ void Projector::autotune(bool f32) {
         // gather policy 2: per-thread async copies into the stage (FP32 steps)
         {0, 12 * 1024, 128, 2, 0, 3}, {0, 20 * 1024, 128, 2, 0, 3}, {0, 24 * 1024, 128, 2, 0, 3},
         {0, 32 * 1024, 256, 2, 0, 4},
-        // the vec engine (FP32 steps): nonzeros per lane x gather cache policy
+        // the vec engine: nonzeros per lane x gather cache policy (FP64 steps: eight only)
         {2, 1, 32, 0, 0, 4}, {2, 1, 32, 1, 0, 4}, {2, 2, 32, 0, 0, 4}, {2, 2, 32, 1, 0, 4},
         {2, 4, 32, 0, 0, 4}, {2, 4, 32, 1, 0, 4}, {2, 8, 32, 0, 0, 4}, {2, 8, 32, 1, 0, 4}};
     constexpr int NC = sizeof(cands) / sizeof(cands[0]);
+    // FP64 steps on the vec engine: only with eight nonzeros per lane, so that the short
+    // rows keep the order of one sequential sum
+    auto vec_ok = [&](int i) { return f32 || cands[i].stage == 8; };
     cudaEvent_t e0, e1;
     PDFP_CK(cudaEventCreate(&e0));
     PDFP_CK(cudaEventCreate(&e1));
@@ -1063,7 +1070,7 @@ void Projector::autotune(bool f32) {
             sides[i].max_blocks = cands[i].max_blocks;
             sides[i].half_red = cands[i].half_red != 0;
             if (cands[i].engine == 2) {
-                if (!f32) continue;  // FP32 steps only
+                if (!vec_ok(i)) continue;
                 sides[i].lane_nnz = cands[i].stage;
             }
             prepare_side(sides[i], primal, f32);
@@ -1077,7 +1084,7 @@ void Projector::autotune(bool f32) {
         for (int sweep = 0; sweep < 2; ++sweep) {
             for (int i = 0; i < NC; ++i) {
                 if (cands[i].l2 == 2 && !f32) continue;  // FP64 steps have no async policy
-                if (cands[i].engine == 2 && !f32) continue;
+                if (cands[i].engine == 2 && !vec_ok(i)) continue;
                 best_ms[i] = std::min(best_ms[i], time_side(sides[i], primal,
                                                             primal ? dual0 : (f32 ? p32_ : p64_)));
             }

@@ -88,7 +88,7 @@ class Projector {
     // One side of the PDHG step: its tile geometry, block size and tiling.
     struct StepSide {
         int engine = 0;  // 0: tile engine (tile_spmv.cuh), 1: flat engine (flat_spmv.cuh),
-                         // 2: vec engine (vec_spmv.cuh; FP32 steps)
+                         // 2: vec engine (vec_spmv.cuh)
         int qpt = 2;     // flat engine: quads (4 nonzeros) per thread and tile, 1 or 2
         int lane_nnz = 4;  // vec engine: target nonzeros per lane of a row
         VecDev vec{};      // vec engine: its items

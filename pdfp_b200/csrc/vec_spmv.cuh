@@ -23,9 +23,12 @@
 // items w, w + W, w + 2W, ... of the list (W warps in the grid): a static
 // longest-first schedule.  Against the tile engine it trades the staged,
 // pipelined tiles for more gathers in flight per SM and no hand-offs; which is
-// faster depends on the matrix, so the autotuner times it with the others.  The
-// FP32 steps only: its lane sums change the order in which a row's terms are
-// added, which the FP64 form (that takes the oracle's steps) does not allow.
+// faster depends on the matrix, so the autotuner times it with the others.  FP64 steps
+// take it with eight nonzeros per lane only: a row of up to eight is then one sequential
+// sum in storage order, a longer one the sum of its lanes' (an order that depends on its
+// length alone).  On a 300,000 x 600,000 zipf-lp matrix with 6M nonzeros the FP64 passes
+// take 33 (A') and 38 us (A) against the tile engine's 47 and 48, 200 iterations 13.0 ms
+// against 17.8; at 40,000 x 80,000 with 1M, 14.1 and 14.2 us against 16.5 and 15.4.
 #pragma once
 #include "common.cuh"
 #include "layout.hpp"
@@ -39,6 +42,12 @@ constexpr int kVecThreads = 256;  // 8 warps per block
 // resident blocks per SM the step kernels are compiled for (48 registers a thread: at 6
 // blocks and 40 registers the A'-side kernel spills and runs slower)
 constexpr int kVecMinBlocks = PDFP_VEC_MIN_BLOCKS;
+#ifndef PDFP_VEC_MIN_BLOCKS64
+#define PDFP_VEC_MIN_BLOCKS64 4
+#endif
+// FP64 steps: 64 registers, no spills (with three blocks the A' side of the zipf-lp matrix
+// above takes 41 us)
+constexpr int kVecMinBlocks64 = PDFP_VEC_MIN_BLOCKS64;
 
 template <class Op>
 __device__ __forceinline__ void vec_rows(const VecDev& s, const Op& op, const VecItem& m,
@@ -179,7 +188,8 @@ __device__ __forceinline__ void vec_pass(const VecDev& s, const Op& op) {
 }
 
 template <class Op>
-__global__ void __launch_bounds__(kVecThreads, kVecMinBlocks) vec_spmv_kernel(const VecDev s, const Op op) {
+__global__ void __launch_bounds__(kVecThreads, sizeof(typename Op::AT) == 8 ? kVecMinBlocks64 : kVecMinBlocks)
+    vec_spmv_kernel(const VecDev s, const Op op) {
     vec_pass<Op>(s, op);
 }
 

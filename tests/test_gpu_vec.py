@@ -167,3 +167,25 @@ def test_vec_batch_members_equal_single_handles(oracle, monkeypatch, lane_nnz):
         assert s.solve(prm, 1.0) == st[p], p
         assert s.total_count == counts[p], p
         assert np.array_equal(s.pdhg_x, b.get(p, "pdhg_x")), p
+
+
+def test_fp64_autotuned_steps_match_the_oracle(oracle, monkeypatch):
+    """FP64 steps with the autotuner on (the vec engine among its candidates, eight nonzeros
+    per lane), per-step launches: 400 steps on Zipf rows of 1 to several thousand nonzeros
+    stay within 1e-10 of the oracle (rounding of about 1e-16 a step, not expanded)."""
+    monkeypatch.setenv("PDFP_AUTOTUNE", "1")
+    monkeypatch.setenv("PDFP_RESIDENT", "0")
+    milp, _ = synthetic.zipf_lp(seed=6, m=4001, n=15007, nnz=180_001)
+    sc, is_eq, is_int, w = oracle.projector_inputs(milp)
+    probs = (sc.A, sc.con_ub, is_eq, is_int, sc.var_lb, sc.var_ub, w)
+    xt = np.zeros(len(milp.c))
+    xt[milp.int_idx] = np.round(np.random.default_rng(3).random(len(milp.int_idx)))
+    prm = SolverParameters(eps_optimal_relative=1e-9, eps_feasible_relative=1e-9, iteration_limit=400)
+    s, o = gpu.PDFPState(*probs, precision="fp64"), oracle.OracleSolvers.PDFPState(*probs)
+    for h in (s, o):
+        h.set_target(xt / sc.D_c)
+        h.solve(prm, 1.0)
+    assert s.total_count == o.total_count == 400
+    for name in ("pdhg_x", "pdhg_y", "pdhg_z", "current_x", "current_z"):
+        a, b = s.get(name), o.get(name)
+        assert np.linalg.norm(a - b) <= 1e-10 * max(1.0, np.linalg.norm(b)), name
