@@ -456,9 +456,9 @@ struct ClusterForm {
     int n_warps = 1;           // warps per block: the most slices of one
     bool ready() const { return r.n_blocks > 0; }
 
-    // Lays every member out, if each fits a cluster; stream-ordered.
+    // Lays every member out, if each fits a cluster; the values follow with fill().
     template <class P>
-    void prepare(const DeviceMatrix& M, DeviceArena& ar, int max_smem_block, cudaStream_t stream) {
+    void prepare(const DeviceMatrix& M, DeviceArena& ar, int max_smem_block) {
         using T = typename P::T;
         if (tried) return;
         tried = true;
@@ -468,10 +468,14 @@ struct ClusterForm {
             if (!M.make_cluster(ar, c, sizeof(T), kCluWarps, cap, f, n_warps)) continue;
             n_ranks = c;
             if (c == 1) set_attr(cluster_windows_kernel<P, false>, cap); else set_attr(cluster_windows_kernel<P, true>, cap);
-            M.fill_resident(ar, f, std::is_same<T, float>::value, stream);
             r = f;
             return;
         }
+    }
+    // The matrix's values into the layout, once; stream-ordered.
+    template <class P>
+    void fill(const DeviceMatrix& M, DeviceArena& ar, cudaStream_t stream) {
+        if (ready() && !r.t.val) M.fill_resident(ar, r, std::is_same<typename P::T, float>::value, stream);
     }
 
     template <class P>

@@ -800,7 +800,8 @@ template <typename T>
 ClusterForm& Projector::ensure_cluster() {
     std::shared_ptr<ClusterForm>& f = std::is_same<T, float>::value ? clu32_ : clu64_;
     if (!f) f = std::make_shared<ClusterForm>();
-    f->prepare<PdfpCluster<T>>(M_, ar_, max_smem_block_, stream_);
+    f->prepare<PdfpCluster<T>>(M_, ar_, max_smem_block_);
+    f->fill<PdfpCluster<T>>(M_, ar_, stream_);
     return *f;
 }
 

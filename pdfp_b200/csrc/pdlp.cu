@@ -272,7 +272,7 @@ struct LpCluster : LpResident<TT> {
 
 // ---- a small LP's whole solve in one launch ---------------------------------------------
 //
-// As for the projector (tiny_solve_kernel, pdfp.cu): one block runs whole evaluation
+// With cuPDLPx termination, whose ray passes the cluster form lacks: one block runs whole evaluation
 // windows of pdlp_solve! (src/pdlp.jl:332-370) -- step 1, the evaluation after a
 // restart, steps 2 .. freq-1, step freq, the full evaluation, the cuPDLPx ray passes,
 // the controller and the restart copy -- until the LP stops, asks for the FP64 polish,
@@ -474,6 +474,10 @@ class LpSolver {
             const char* te = std::getenv("PDFP_TINY");
             tiny_ = !(te && te[0] == '0') && static_cast<int64_t>(A.m) + A.n <= 4096 &&
                     M_.L.NNZ <= (1 << 16);
+            if (tiny_ && !cupdlpx_) {  // whole windows in a cluster, or else as a larger LP
+                if (f32_) clu32_.prepare<LpCluster<float>>(M_, ar_, max_smem_); else clu64_.prepare<LpCluster<double>>(M_, ar_, max_smem_);
+                tiny_ = (f32_ ? clu32_ : clu64_).ready();
+            }
         }
         m_ = A.m;
         n_ = A.n;
@@ -717,8 +721,9 @@ void LpSolver::launch_tiny_solve() {
     LpVecs<T>* vp = nullptr;
     if constexpr (std::is_same<T, float>::value) vp = &v32_; else vp = &v64_;
     ClusterForm& cf = std::is_same<T, float>::value ? clu32_ : clu64_;
-    if (!cupdlpx_) cf.template prepare<LpCluster<T>>(M_, ar_, max_smem_, stream_);
+    if (!cupdlpx_) cf.template prepare<LpCluster<T>>(M_, ar_, max_smem_);
     if (cf.ready()) {
+        cf.template fill<LpCluster<T>>(M_, ar_, stream_);
         LpCluster<T> prob;
         static_cast<LpResident<T>&>(prob) =
             LpResident<T>{*vp, st_, std::is_same<T, float>::value ? MODE_FP32 : MODE_FP64, err_};
