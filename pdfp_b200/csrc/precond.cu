@@ -301,6 +301,155 @@ void scale_uploaded(const DeviceMatrix& M, DeviceArena& ar, int32_t ruiz_iterati
     PDFP_CK(cudaGetLastError());
 }
 
+// ---- A' on the device, for scale_problem of a matrix that is not small --------------
+//
+// scale_problem needs A' only to read each column's entries in ascending row order.  The
+// host's transposition (a pass of scattered writes over every nonzero) and its second
+// upload took most of the call at 500k nonzeros; here the device counts the columns'
+// entries, scans the counts, drops every entry into its column and orders each column by
+// row.  Below kDeviceTransposeNnz the host's way costs less than these launches.
+constexpr int64_t kDeviceTransposeNnz = 1 << 16;
+constexpr int kScanThreads = 1024;
+constexpr int32_t kShortColumn = 64;  // ordered by one thread; a longer one by a block
+
+__global__ void count_columns_kernel(const int32_t* __restrict__ ci, int64_t nnz, int32_t* __restrict__ count) {
+    for (int64_t e = blockIdx.x * int64_t(256) + threadIdx.x; e < nnz; e += int64_t(gridDim.x) * 256)
+        atomicAdd(count + ci[e], 1);
+}
+// rp[0 .. n] = exclusive sums of count[0 .. n); cursor = rp; one block
+__global__ void __launch_bounds__(kScanThreads) scan_columns_kernel(const int32_t* __restrict__ count, int32_t n,
+                                                                    int32_t* __restrict__ rp, int32_t* __restrict__ cursor) {
+    __shared__ int32_t warp_sum[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int32_t carry = 0;
+    for (int64_t base = 0; base < n; base += kScanThreads) {
+        const int64_t j = base + threadIdx.x;
+        const int32_t x = j < n ? count[j] : 0;
+        int32_t v = x;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int32_t y = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= o) v += y;
+        }
+        if (lane == 31) warp_sum[warp] = v;
+        __syncthreads();
+        if (warp == 0) {
+            int32_t w = warp_sum[lane];
+            for (int o = 1; o < 32; o <<= 1) {
+                const int32_t y = __shfl_up_sync(0xffffffffu, w, o);
+                if (lane >= o) w += y;
+            }
+            warp_sum[lane] = w;
+        }
+        __syncthreads();
+        const int32_t before = carry + (warp > 0 ? warp_sum[warp - 1] : 0) + v - x;
+        if (j < n) {
+            rp[j] = before;
+            cursor[j] = before;
+        }
+        carry += warp_sum[31];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) rp[n] = carry;
+}
+// every entry into its column, in any order: its row and its place in A
+__global__ void fill_columns_kernel(const int32_t* __restrict__ rp_a, const int32_t* __restrict__ ci_a, int32_t m,
+                                    int32_t* __restrict__ cursor, int2* __restrict__ entry) {
+    const int lane = threadIdx.x & 31;
+    for (int32_t i = (blockIdx.x * 256 + threadIdx.x) >> 5; i < m; i += (gridDim.x * 256) >> 5)
+        for (int32_t e = rp_a[i] + lane; e < rp_a[i + 1]; e += 32) entry[atomicAdd(cursor + ci_a[e], 1)] = make_int2(i, e);
+}
+// columns in ascending row order: ci_t the rows, v_t the values.  A column holds a row at
+// most once, so an entry's place is the number of smaller rows.
+__global__ void order_short_columns_kernel(const int32_t* __restrict__ rp_t, int32_t n, const int2* __restrict__ entry,
+                                           const double* __restrict__ v_a, int32_t* __restrict__ ci_t,
+                                           double* __restrict__ v_t) {
+    for (int32_t j = blockIdx.x * 256 + threadIdx.x; j < n; j += gridDim.x * 256) {
+        const int32_t b = rp_t[j], len = rp_t[j + 1] - b;
+        if (len > kShortColumn) continue;
+        for (int32_t k = 0; k < len; ++k) {
+            const int2 x = entry[b + k];
+            int32_t at = b;
+            for (int32_t q = 0; q < len; ++q) at += entry[b + q].x < x.x ? 1 : 0;
+            ci_t[at] = x.x;
+            v_t[at] = v_a[x.y];
+        }
+    }
+}
+__global__ void __launch_bounds__(256) order_long_columns_kernel(const int32_t* __restrict__ rp_t, int32_t n,
+                                                                 const int2* __restrict__ entry,
+                                                                 const double* __restrict__ v_a,
+                                                                 int32_t* __restrict__ ci_t, double* __restrict__ v_t) {
+    __shared__ int32_t rows[1024];
+    for (int32_t j = blockIdx.x; j < n; j += gridDim.x) {
+        const int32_t b = rp_t[j], len = rp_t[j + 1] - b;
+        if (len <= kShortColumn) continue;  // the same for the whole block
+        for (int32_t k0 = 0; k0 < len; k0 += 256) {
+            const int32_t k = k0 + threadIdx.x;
+            const int2 x = k < len ? entry[b + k] : make_int2(0, 0);
+            int32_t at = b;
+            for (int32_t q0 = 0; q0 < len; q0 += 1024) {
+                const int32_t c = len - q0 < 1024 ? len - q0 : 1024;
+                __syncthreads();
+                for (int32_t q = threadIdx.x; q < c; q += 256) rows[q] = entry[b + q0 + q].x;
+                __syncthreads();
+                if (k < len)
+                    for (int32_t q = 0; q < c; ++q) at += rows[q] < x.x ? 1 : 0;
+            }
+            if (k < len) {
+                ci_t[at] = x.x;
+                v_t[at] = v_a[x.y];
+            }
+        }
+    }
+}
+
+// build_layout's checks of one problem, without its layout.
+static std::string check_csr(const pdfp_csr& A, const int32_t* rp) {
+    if (A.m < 0 || A.n < 0) return "negative dimension";
+    if (A.m > 0 && !A.row_ptr) return "null row_ptr";
+    if (A.m > 0 && rp[0] != 0) return "row_ptr[0] must be 0";
+    for (int32_t i = 0; i < A.m; ++i) {
+        if (rp[i + 1] < rp[i]) return "row_ptr is not monotone";
+        for (int32_t q = rp[i]; q < rp[i + 1]; ++q) {
+            if (A.col_idx[q] < 0 || A.col_idx[q] >= A.n) return "column index out of range";
+            if (q > rp[i] && A.col_idx[q] <= A.col_idx[q - 1])
+                return "column indices must be strictly ascending within a row";
+            if (!std::isfinite(A.val[q])) return "non-finite matrix value";
+        }
+    }
+    if (A.m > 0 && rp[A.m] > 0x7fffff00LL) return "problem too large for int32 indexing";
+    return "";
+}
+
+// The caller's matrix and its transpose on the device, on the default stream.
+static void upload_transposed(const pdfp_csr& A, DeviceArena& ar, DeviceMatrix& M) {
+    const int32_t m = A.m, n = A.n;
+    const int64_t nnz = A.row_ptr[m];
+    M.L.K = 1;
+    M.L.M = m;
+    M.L.N = n;
+    M.L.NNZ = nnz;
+    M.rp_a = ar.alloc<int32_t>(static_cast<size_t>(m) + 1);
+    M.ci_a = ar.alloc<int32_t>(nnz);
+    M.v64_a = ar.alloc<double>(nnz);
+    M.rp_t = ar.alloc<int32_t>(static_cast<size_t>(n) + 1);
+    M.ci_t = ar.alloc<int32_t>(nnz);
+    M.v64_t = ar.alloc<double>(nnz);
+    int32_t* const count = ar.alloc<int32_t>(n);  // zero-filled
+    int32_t* const cursor = ar.alloc<int32_t>(n);
+    int2* const entry = ar.alloc<int2>(nnz);
+    PDFP_CK(cudaMemcpyAsync(M.rp_a, A.row_ptr, sizeof(int32_t) * (size_t(m) + 1), cudaMemcpyHostToDevice, 0));
+    PDFP_CK(cudaMemcpyAsync(M.ci_a, A.col_idx, sizeof(int32_t) * nnz, cudaMemcpyHostToDevice, 0));
+    const int be = static_cast<int>(std::min<int64_t>((nnz + 255) / 256, 8192)), bn = blocks_for(n);
+    count_columns_kernel<<<be, 256>>>(M.ci_a, nnz, count);
+    scan_columns_kernel<<<1, kScanThreads>>>(count, n, M.rp_t, cursor);
+    fill_columns_kernel<<<be, 256>>>(M.rp_a, M.ci_a, m, cursor, entry);
+    PDFP_CK(cudaMemcpyAsync(M.v64_a, A.val, sizeof(double) * nnz, cudaMemcpyHostToDevice, 0));
+    order_short_columns_kernel<<<bn, 256>>>(M.rp_t, n, entry, M.v64_a, M.ci_t, M.v64_t);
+    order_long_columns_kernel<<<std::min(n, 4 * 148), 256>>>(M.rp_t, n, entry, M.v64_a, M.ci_t, M.v64_t);
+    PDFP_CK(cudaGetLastError());
+}
+
 void scale_problem_device(const pdfp_csr& A, const double* c, const double* var_lb,
                           const double* var_ub, const double* con_lb, const double* con_ub,
                           int32_t ruiz_iterations, double alpha, bool rescale, double* val_out,
@@ -311,10 +460,16 @@ void scale_problem_device(const pdfp_csr& A, const double* c, const double* var_
     const int32_t m = A.m, n = A.n;
     ProblemIn in{m, n, m > 0 ? A.row_ptr : &zero_rp, A.col_idx, A.val, nullptr};
     DeviceMatrix M;
-    std::string msg = build_layout({in}, false, M.L);
-    if (!msg.empty()) throw Error(E_INVALID, msg);
     DeviceArena ar;
-    M.upload(ar, false);
+    if (m > 0 && n > 0 && A.row_ptr && A.row_ptr[m] >= kDeviceTransposeNnz) {
+        const std::string msg = check_csr(A, A.row_ptr);
+        if (!msg.empty()) throw Error(E_INVALID, msg);
+        upload_transposed(A, ar, M);
+    } else {
+        std::string msg = build_layout({in}, false, M.L);
+        if (!msg.empty()) throw Error(E_INVALID, msg);
+        M.upload(ar, false);
+    }
     // inputs in one block: c, lb, ub (n each), con_lb, con_ub (m each), then the outputs,
     // D_c, D_r and the two scales
     const int64_t tot = 3 * int64_t(n) + 2 * int64_t(m);

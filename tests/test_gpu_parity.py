@@ -406,3 +406,23 @@ def test_whole_window_kernel_staged_equals_unstaged(oracle, monkeypatch, precisi
     for a, bb in zip(x1, x0):
         assert np.array_equal(a, bb)
     assert np.array_equal(y1, y0)
+
+
+def test_scale_problem_transposed_on_the_device(oracle):
+    """At least 65,536 nonzeros: A' is built on the device.  Columns without entries, of one
+    entry, at the edges of a thread's (64) and a block's chunk (1,024) of rows, and a dense
+    one: factors and values bit for bit."""
+    rng = np.random.default_rng(12)
+    m, lens = 2500, [0, 1, 63, 64, 65, 255, 256, 257, 1023, 1024, 1025, 2500] + [40] * 1500
+    cols = [np.sort(rng.choice(m, size=k, replace=False)) for k in lens]
+    A = sp.csc_matrix((rng.uniform(-3.0, 3.0, size=sum(lens)), np.concatenate(cols),
+                       np.concatenate([[0], np.cumsum(lens)])), shape=(m, len(lens))).tocsr()
+    A = A[:, rng.permutation(len(lens))].tocsr()
+    A.sort_indices()
+    assert A.nnz >= 1 << 16
+    n = len(lens)
+    args = (A, rng.uniform(-1, 1, n), np.zeros(n), np.ones(n), np.full(m, -np.inf), rng.uniform(0.5, 2.0, m))
+    g, o = gpu.scale_problem(*args), oracle.scale_problem(*args)
+    assert np.array_equal(g.A.data, o.A.data)
+    for name in ("D_r", "D_c", "c", "var_ub", "con_ub"):
+        assert np.array_equal(getattr(g, name), getattr(o, name)), name
