@@ -153,7 +153,8 @@ struct ResSide {
     uint32_t idx, val, prod, slices, lane, longs, vec, slots, arr, par;
     int32_t n_slices, n_elem, row0, rows;
     int32_t first_warp;    // the warp that sums slice 0
-    int32_t n_par;         // columns: the parameter entries of both sides (they adjoin)
+    uint32_t par_all;      // the parameter entries of both sides (they adjoin)
+    int32_t n_par;
 };
 
 // After 64 fruitless looks: whether the wait is over for good.
@@ -189,6 +190,18 @@ __device__ __noinline__ int32_t res_long(unsigned char* sm, const ResSide<T>& s,
     for (int32_t e = 0; e < l.np; ++e) tot += slots[l.slot0 + e];
     acc = static_cast<T>(tot);
     return l.row;
+}
+
+// The weights k / (k + 1) of step k of every instance of the block.
+template <typename T>
+__device__ __forceinline__ void res_weights(unsigned char* sm, const ResSide<T>& s, int32_t k, int t, int n) {
+    ResPar<T>* par = reinterpret_cast<ResPar<T>*>(sm + s.par_all);
+    for (int32_t p = t; p < s.n_par; p += n) {
+        const double kk = static_cast<double>(par[p].inner + k);
+        const double weight = kk / (kk + 1.0);
+        par[p].weight[k & 1] = static_cast<T>(weight);
+        par[p].omwt[k & 1] = static_cast<T>(1.0 - weight);
+    }
 }
 
 // The sum of a lane's products, in order.
@@ -238,13 +251,30 @@ __device__ __forceinline__ void res_pass(const P& prob, unsigned char* sm, const
     const int32_t* idx = reinterpret_cast<const int32_t*>(sm + s.idx);
     const T* val = reinterpret_cast<const T*>(sm + s.val);
     T* prod = reinterpret_cast<T*>(sm + s.prod);
-    // the warp's first slice and its lanes' rows, read before the wait
+    // the warp's first slice, its lanes' rows with their vectors and the step's parameters,
+    // read before the wait
     int32_t q = (warp + kResThreads / 32 - s.first_warp) % (kResThreads / 32), r = -1;
-    ResSlice m;
+    ResSlice m{};
+    StepParams<T> p{};
+    int32_t eq_end = 0;
+    bool act = false;
+    T in[P::NCV];
+    auto read_vecs = [&](int32_t row) {
+        const T* pv = reinterpret_cast<const T*>(sm + s.vec) + row;
+#pragma unroll
+        for (int e = 0; e < P::NCV; ++e)
+            if (e < P::NRV || !is_row) in[e] = pv[e * s.rows];
+    };
     auto next_slice = [&]() {
         if (q >= s.n_slices) return;
         m = reinterpret_cast<const ResSlice*>(sm + s.slices)[q];
         r = reinterpret_cast<const int32_t*>(sm + s.lane)[q * 32 + lane];
+        if (m.slot >= 0) r = 0;
+        const ResPar<T>& pr = reinterpret_cast<const ResPar<T>*>(sm + s.par)[m.inst];
+        p = StepParams<T>{pr.tau, pr.sigma, T(0), T(0), pr.omega, pr.omw};
+        eq_end = pr.eq_end;
+        act = pr.act != 0;
+        read_vecs(r < 0 ? 0 : r);
     };
     next_slice();
     if (lane == 0 && static_cast<int32_t>(threadIdx.x) < s.n_elem) {
@@ -257,15 +287,6 @@ __device__ __forceinline__ void res_pass(const P& prob, unsigned char* sm, const
             res_get(s.in + c, x, t);
             if (t == want) break;
             if ((++spins & 63u) == 0) off = res_gave_up(dead, prob.errp, t0);
-        }
-    }
-    if (warp == kResThreads / 32 - 1 && !is_row) {  // the step's weights, k / (k + 1)
-        ResPar<T>* par = reinterpret_cast<ResPar<T>*>(sm + s.par);
-        for (int32_t p = lane; p < s.n_par; p += 32) {
-            const double kk = static_cast<double>(par[p].inner + k);
-            const double weight = kk / (kk + 1.0);
-            par[p].weight[k & 1] = static_cast<T>(weight);
-            par[p].omwt[k & 1] = static_cast<T>(1.0 - weight);
         }
     }
     __syncwarp();
@@ -299,25 +320,15 @@ __device__ __forceinline__ void res_pass(const P& prob, unsigned char* sm, const
     __syncthreads();
 #pragma unroll 1
     while (q < s.n_slices) {
-        const ResPar<T>& pr = reinterpret_cast<const ResPar<T>*>(sm + s.par)[m.inst];
-        if (pr.act) {
+        if (act) {
             const bool piece = m.slot >= 0;
-            if (piece) r = 0;
-            T* pv = reinterpret_cast<T*>(sm + s.vec) + (r < 0 ? 0 : r);
-            const StepParams<T> p{pr.tau, pr.sigma, pr.weight[k & 1], pr.omwt[k & 1], pr.omega, pr.omw};
-            T in[P::NCV], acc;
-#pragma unroll
-            for (int e = 0; e < P::NCV; ++e)
-                if (e < P::NRV || !is_row) in[e] = pv[e * s.rows];
-            acc = res_sum(prod + m.off + lane, m.shape >> 3);
+            const ResPar<T>& pr = reinterpret_cast<const ResPar<T>*>(sm + s.par)[m.inst];
+            p.weight = pr.weight[k & 1];  // written in the pass before
+            p.omwt = pr.omwt[k & 1];
+            T acc = res_sum(prod + m.off + lane, m.shape >> 3);
             if (piece) {
                 r = res_long<T>(sm, s, m, q, acc);
-                if (r >= 0) {
-                    pv = reinterpret_cast<T*>(sm + s.vec) + r;
-#pragma unroll
-                    for (int e = 0; e < P::NCV; ++e)
-                        if (e < P::NRV || !is_row) in[e] = pv[e * s.rows];
-                }
+                if (r >= 0) read_vecs(r);
             } else if (m.shape & 7) {
                 const int G = 1 << (m.shape & 7);
 #pragma unroll 1
@@ -326,11 +337,12 @@ __device__ __forceinline__ void res_pass(const P& prob, unsigned char* sm, const
             }
             if (r >= 0) {
                 const int32_t i = s.row0 + r;
+                T* pv = reinterpret_cast<T*>(sm + s.vec) + r;
                 if (is_row) {
                     T in3[P::NRV];
 #pragma unroll
                     for (int e = 0; e < P::NRV; ++e) in3[e] = in[e];
-                    res_put(s.out + i, prob.template row<MAJOR>(p, i < pr.eq_end, i, in3, pv, s.rows, acc), k + 1);
+                    res_put(s.out + i, prob.template row<MAJOR>(p, i < eq_end, i, in3, pv, s.rows, acc), k + 1);
                 } else {
                     const typename P::X x = prob.col_x(p, in, acc);
                     res_put(s.out + i, x.rx, k);
@@ -342,6 +354,7 @@ __device__ __forceinline__ void res_pass(const P& prob, unsigned char* sm, const
         q += kResThreads / 32;
         next_slice();
     }
+    if (is_row && warp == kResThreads / 32 - 1) res_weights<T>(sm, s, k + 1, lane, 32);  // before the next barrier
 }
 
 // Steps i0 .. i1 of every active instance (K of them), i0 >= 1; step i1 is major.
@@ -363,11 +376,11 @@ __global__ void __launch_bounds__(kResThreads, 1)
         if (threadIdx.x == 0) {
             sides[0] = ResSide<T>{wz, wx, o.idx_t, o.val_t, o.prod_t, o.slice_t, o.lane_t, o.long_t, o.col,
                                   o.slots_t, o.arr_t, o.par_t, bt.n_slices, bt.n_elem, bt.row0,
-                                  bt.row1 - bt.row0, 0, bt.n_inst + ba.n_inst};
+                                  bt.row1 - bt.row0, 0, o.par_t, bt.n_inst + ba.n_inst};
             // the row slices go to the warps after those of the column slices
             sides[1] = ResSide<T>{wx, wz, o.idx_a, o.val_a, o.prod_a, o.slice_a, o.lane_a, o.long_a, o.row,
                                   o.slots_a, o.arr_a, o.par_a, ba.n_slices, ba.n_elem, ba.row0,
-                                  ba.row1 - ba.row0, bt.n_slices % (kResThreads / 32), 0};
+                                  ba.row1 - ba.row0, bt.n_slices % (kResThreads / 32), o.par_t, bt.n_inst + ba.n_inst};
         }
         __syncthreads();
 #pragma unroll 1
@@ -428,6 +441,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
             }
         }
     }
+    res_weights<T>(sm, sides[0], i0, threadIdx.x, kResThreads);
     __syncthreads();
     bool off = false;
 #pragma unroll 1
