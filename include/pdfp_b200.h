@@ -251,8 +251,8 @@ PDFP_API int pdfp_set_polish(pdfp_handle* h, int32_t stall_evaluations, double f
  * roundings in the same order, so results do not depend on the policy).
  * The steps may also run on the vec engine (warps over rows read straight
  * from the CSR arrays, lanes per row by row length; threads per role 32, "stage
- * bytes" its target nonzeros per lane 1, 2, 4 or 8 -- FP64 steps: 8, and only where
- * the autotuner picks it; gather policy 0 or 1).
+ * bytes" its target nonzeros per lane 1, 2, 4 or 8 -- FP64 steps: 8, where the
+ * autotuner picks it or PDFP_TUNING pins it; gather policy 0 or 1).
  * PDFP_AUTOTUNE=0 / =1 switches it off / on regardless of size, and
  * PDFP_STEP_ENGINE=tile / =flat / =flat1 / =vec fixes the engine with its default
  * settings (flat1: the flat engine's one-quad-per-thread variant; vec: the FP32

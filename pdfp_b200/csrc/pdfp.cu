@@ -467,8 +467,10 @@ Projector::Projector(const std::vector<ProblemData>& probs, int precision) : pre
     }
     M_.upload(ar_, precision_ == PDFP_MIXED);
     // Small members (every one at most kTinyMaxDim rows + columns and
-    // kTinyMaxNnz nonzeros; PDFP_TINY=0 switches this off): the minor steps of a
-    // window run in one launch, one block per member.
+    // kTinyMaxNnz nonzeros and fitting a cluster; PDFP_TINY=0 switches this off): whole
+    // windows run in one launch, one thread-block cluster per member
+    // (cluster_windows.cuh); in timing mode, or for a polish whose FP64 form does not
+    // fit, the minor steps of a captured window in one block per member (tiny_steps.cuh).
     {
         const char* te = std::getenv("PDFP_TINY");
         tiny_ = !(te && te[0] == '0') && K_ <= 65535;
@@ -695,7 +697,7 @@ Projector::Projector(const std::vector<ProblemData>& probs, int precision) : pre
     // PDFP_TUNING="s,t,l,s,t,l" pins both sides' step kernels of this precision
     // (A' then A: stage bytes, threads per role -- 0: flat engine, whose stage
     // bytes tell its variant; 32: vec engine, whose "stage bytes" are its nonzeros
-    // per lane, FP32 steps only -- and the L2-only gather flag), as pdfp_get_tuning
+    // per lane, for FP64 steps eight -- and the L2-only gather flag), as pdfp_get_tuning
     // reports them; the tuner does not run.
     bool pinned = false;
     if (const char* pt = std::getenv("PDFP_TUNING")) {
@@ -716,7 +718,7 @@ Projector::Projector(const std::vector<ProblemData>& probs, int precision) : pre
                 const int* c = v + 3 * k;
                 if (c[1] != 0 && c[1] != 32 && c[1] != 128 && c[1] != 256)
                     throw Error(E_INVALID, "PDFP_TUNING: threads per role must be 0, 32, 128 or 256");
-                if (c[1] == 32) {  // the vec engine: FP32 steps; the FP64 steps keep their default
+                if (c[1] == 32) {  // the vec engine; FP64 steps: of an FP64 handle, eight per lane
                     if (c[0] != 1 && c[0] != 2 && c[0] != 4 && c[0] != 8)
                         throw Error(E_INVALID, "PDFP_TUNING: the vec engine's nonzeros per lane must "
                                                "be 1, 2, 4 or 8");
@@ -724,7 +726,7 @@ Projector::Projector(const std::vector<ProblemData>& probs, int precision) : pre
                         throw Error(E_INVALID, "PDFP_TUNING: the vec engine's gather policy must be 0 or 1");
                     if (v[10 + k] != 0)
                         throw Error(E_INVALID, "PDFP_TUNING: the vec engine has no reducers (0)");
-                    if (f == 1) continue;
+                    if (f == 1 && (precision_ != PDFP_FP64 || c[0] != 8)) continue;
                     q.engine = 2;
                     q.lane_nnz = c[0];
                     q.gather_l2 = c[2];

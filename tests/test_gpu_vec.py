@@ -189,3 +189,24 @@ def test_fp64_autotuned_steps_match_the_oracle(oracle, monkeypatch):
     for name in ("pdhg_x", "pdhg_y", "pdhg_z", "current_x", "current_z"):
         a, b = s.get(name), o.get(name)
         assert np.linalg.norm(a - b) <= 1e-10 * max(1.0, np.linalg.norm(b)), name
+
+
+@pytest.mark.parametrize("lane_nnz,runs", [(8, True), (4, False)])
+def test_fp64_handle_takes_the_pinned_vec_engine(oracle, monkeypatch, lane_nnz, runs):
+    """A pinned vec engine with eight nonzeros per lane is what an FP64 handle then runs and
+    reports (other widths leave its steps on the default engine); 200 steps stay within 1e-10 of
+    the oracle."""
+    milp, _ = synthetic.zipf_lp(seed=9, m=2003, n=5007, nnz=60_001)
+    sc, is_eq, is_int, w = oracle.projector_inputs(milp)
+    probs = (sc.A, sc.con_ub, is_eq, is_int, sc.var_lb, sc.var_ub, w)
+    xt = np.zeros(len(milp.c))
+    monkeypatch.setenv("PDFP_TUNING", f"{lane_nnz},32,0,{lane_nnz},32,1")
+    prm = SolverParameters(eps_optimal_relative=1e-9, eps_feasible_relative=1e-9, iteration_limit=200)
+    s, o = gpu.PDFPState(*probs, precision="fp64"), oracle.OracleSolvers.PDFPState(*probs)
+    assert [t == 32 for t in (s.tuning()[1], s.tuning()[4])] == [runs, runs]
+    for h in (s, o):
+        h.set_target(xt)
+        h.solve(prm, 1.0)
+    for name in ("pdhg_x", "pdhg_y", "current_z"):
+        a, b = s.get(name), o.get(name)
+        assert np.linalg.norm(a - b) <= 1e-10 * max(1.0, np.linalg.norm(b)), name
