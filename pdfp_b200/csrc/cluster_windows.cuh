@@ -57,9 +57,8 @@ __device__ __forceinline__ void cluster_put(uint32_t a, int32_t v) {
     asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
 }
 // All threads of the cluster meet; what each wrote before (shared memory of any of its
-// blocks, global memory) is visible to all after.  The compiler's own barrier functions:
-// inline assembly could be duplicated into the branches before it, and a warp's lanes
-// would then arrive at different copies of the barrier, which the hardware rejects.
+// blocks, global memory) is visible to all after.  The compiler's own barrier functions,
+// after a warp-wide join: every lane of a warp arrives at the same instruction.
 template <bool CL>
 __device__ __forceinline__ void cluster_meet() {
     if (CL) {

@@ -482,8 +482,8 @@ class LpSolver {
         m_ = A.m;
         n_ = A.n;
         const int e = f32_ ? 4 : 8;
-        // the step tilings serve the captured window only (a small LP runs
-        // lp_tiny_solve_kernel); the evaluation tilings also serve the power iteration
+        // the step tilings serve the captured window only (a small LP runs in a
+        // cluster or in lp_tiny_solve_kernel); the evaluation tilings also serve the power iteration
         // and the initial norms
         if (!tiny_) {
             it_t_ = M_.make_tiling(ar_, true, StageGeom{e, e, e, 5, 1, 24 * 1024, 2048});
@@ -611,7 +611,7 @@ class LpSolver {
     bool cupdlpx_, f32_;
     std::vector<double> D_c_;
     double bound_scale_ = 1.0, objective_scale_ = 1.0;
-    bool tiny_ = false;  // small LP: whole windows in one launch (lp_tiny_solve_kernel)
+    bool tiny_ = false;  // small LP: whole windows in one launch (a cluster, or lp_tiny_solve_kernel)
     int sms_ = 148;
     int max_smem_ = 232448;  // dynamic shared memory a block may opt into
     int32_t m_ = 0, n_ = 0;
@@ -685,16 +685,7 @@ void LpSolver::record(int freq) {
     evals(EVAL_AFTER_RESTART);
     launch_finalize(1, LpController{ev_t_.inst_tile0, d_.part_col, ev_a_.inst_tile0, d_.part_row,
                                     st_, flags_, 0, cupdlpx_ ? 1 : 0}, stream_);
-    if (tiny_ && freq > 2) {
-        // a small LP: steps 2 .. freq-1 in one launch (tiny_steps.cuh)
-        tiny_steps_kernel<LpPrimalOp<T, false, kTinyThreads>, LpDualOp<T, false, kTinyThreads>>
-            <<<1, kTinyThreads, 0, stream_>>>(LpPrimalOp<T, false, kTinyThreads>{v, st_, 0, mode, err_},
-                                              LpDualOp<T, false, kTinyThreads>{v, st_, 0, mode, err_},
-                                              M_.rp_t, M_.ci_t, M_.rp_a, M_.ci_a, M_.col_off,
-                                              M_.row_off, 2, freq);
-        PDFP_CK(cudaGetLastError());
-        step(freq, true);
-    } else if (resident<T>().ready()) {  // steps 2 .. freq with the LP resident on the chip
+    if (resident<T>().ready()) {  // steps 2 .. freq with the LP resident on the chip
         resident<T>().launch(LpResident<T>{v, st_, mode, err_}, 1, 2, freq, stream_);
     } else {
         for (int i = 2; i <= freq - 1; ++i) step(i, false);

@@ -3,9 +3,9 @@
 // scale_problem, src/preconditioner.jl:26-99: ten Ruiz rounds (1/sqrt of the
 // largest |a| per row and column), one Pock-Chambolle pass (1/sqrt of the sum
 // of |a|^alpha per row, |a|^(2-alpha) per column), then the scaled bounds and
-// the optional bound/objective rescaling.  Row maxima and row sums are taken by
-// one thread per row of A (and of A'), summing in ascending index order, so the
-// scaling factors and scaled values are bit-identical to the reference's CPU
+// the optional bound/objective rescaling.  Row sums are taken by one thread per row of
+// A (and of A') in ascending index order, row maxima, which no order changes, by eight
+// lanes, so the scaling factors and scaled values are bit-identical to the reference's CPU
 // arithmetic (Julia walks its CSC matrix column by column, which gives each row
 // sum its terms in ascending column order and each column sum in ascending row
 // order).  The scaled bounds, costs and the optional bound/objective rescaling

@@ -19,8 +19,9 @@
 // tagged entries), a pass that only exchanges 700 gathers per SM 2,300 cycles and one
 // with 3,400 gathers 5,000 (an SM gets about one scattered gather per cycle through).
 // Measured per PDHG iteration (one B200, FP64, whole solves): 4,001 x 10,007 with 100k
-// nonzeros 13.7 -> 4.7 us, 20,000 x 50,000 with 500k 15.4 -> 8.2 us (mixed form 12.8 ->
-// 8.0).  The same passes with a grid barrier after each instead of tagged entries
+// nonzeros 13.7 -> 4.3 us, 20,000 x 50,000 with 500k 15.4 -> 7.8 us (mixed form 12.8 ->
+// 7.8).  What does not depend on the pass is read before the wait (4.7 and 8.2 us when it
+// was read after).  The same passes with a grid barrier after each instead of tagged entries
 // (release, atomic, acquire, then the gathers) took 6.3 and 11 us.
 //
 // The order in which a row's terms are added depends on its length alone (its lanes
@@ -37,11 +38,11 @@
 
 namespace pdfp {
 
-// 16 warps with 128 registers: 1.87 / 3.26 / 3.39 ms for 400 iterations of the models above
+// 16 warps with 128 registers (timed before the reads moved ahead of the wait): 1.87 / 3.26 / 3.39 ms for 400 iterations of the models above
 // (100k FP64, 500k mixed, 500k FP64) against 2.31 / 3.43 / 3.96 with 32 warps, whose passes
 // spill, and 2.08 / 3.63 / 3.74 with 24.
 constexpr int kResThreads = 512;
-constexpr uint64_t kResWaitNs = 2000000000ull;  // a barrier wait longer than 2 s is declared hung
+constexpr uint64_t kResWaitNs = 2000000000ull;  // a wait for an entry longer than 2 s is declared hung
 
 // One entry of a vector that crosses between blocks, with the step it belongs to.
 template <typename T>
