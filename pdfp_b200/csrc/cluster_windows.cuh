@@ -301,6 +301,7 @@ __global__ void __launch_bounds__(kCluThreads, 1)
     extern __shared__ __align__(16) unsigned char sm[];
     __shared__ CluCtl<T> ctl;
     __shared__ double terms[12];
+    __shared__ double ray_terms[3];
     const uint32_t rank = CL ? cluster_rank() : 0u;
     const int p = static_cast<int>(blockIdx.x / n_ranks), warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
     const int32_t c0 = col_off[p], n = col_off[p + 1] - c0, r0 = row_off[p], m = row_off[p + 1] - r0;
@@ -393,8 +394,47 @@ __global__ void __launch_bounds__(kCluThreads, 1)
                 for (int c = 0; c < len; ++c) sum += q[np * c];
                 terms[t] = sum;
             }
+        }
+        if constexpr (P::kRays) {
+            if (which == EVAL_FULL) {
+                // the ray passes: the rays themselves, then their products, both over the
+                // chunks above; the partial sums take the places of the terms'
+                if (rank == 0) prob.rays_begin();
+                cluster_meet<CL>();
+                for (int32_t c = rank * n_warps + warp; c < nc + nr; c += n_ranks * n_warps) {
+                    const int32_t i = kCluEvalRows * (c < nc ? c : c - nc) + (threadIdx.x & 31);
+                    if (c < nc) {
+                        if (i < n) prob.ray_col(c0 + i);
+                        continue;
+                    }
+                    double s = i < m ? prob.ray_row(r0 + i) : 0.0;
+                    __syncwarp();
+#pragma unroll
+                    for (int q = 16; q > 0; q >>= 1) s += __shfl_xor_sync(0xffffffffu, s, q);
+                    if ((threadIdx.x & 31) == 0) cluster_put(to_r + 32u * (c - nc), s);
+                }
+                cluster_meet<CL>();
+                for (int32_t c = rank * n_warps + warp; c < nc + nr; c += n_ranks * n_warps)
+                    if (c < nc)
+                        clu_eval<typename P::RayCol, 2>(prob.ray_col_op(), rp_t, ci_t, c0, c0 + n, c, p, to_c + 64u * c);
+                    else  // no sums: one place that nothing reads
+                        clu_eval<typename P::RayRow, 1>(prob.ray_row_op(), rp_a, ci_a, r0, r0 + m, c - nc, p, to_r + 32u * (c - nc) + 8u);
+                cluster_meet<CL>();
+                if (rank == 0 && threadIdx.x < 3) {
+                    const int t = threadIdx.x, np = t < 2 ? 8 : 4, len = t < 2 ? nc : nr;
+                    const double* q = reinterpret_cast<const double*>(sm + (t < 2 ? o.part_c : o.part_r)) + (t < 2 ? t : 0);
+                    double sum = 0.0;
+                    for (int c = 0; c < len; ++c) sum += q[np * c];
+                    ray_terms[t] = sum;
+                }
+            }
+        }
+        if (rank == 0) {
+            const int t = threadIdx.x;
             __syncthreads();
             if (t == 0) {
+                if constexpr (P::kRays)
+                    if (which == EVAL_FULL) prob.rays_finalize(p, ray_terms);
                 prob.finalize(p, terms, which);
                 const InstState& st = prob.st[p];
                 const StepParams<T> q = step_params<T>(st, 0);

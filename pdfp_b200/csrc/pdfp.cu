@@ -272,6 +272,7 @@ struct WarmStartCopy {  // initial = current (src/pdfp.jl:105-107)
 
 template <typename TT>
 struct PdfpCluster : PdfpResident<TT> {
+    static constexpr bool kRays = false;
     using T = TT;
     using B = PdfpResident<TT>;
     using EvalCol = EvalColOp<T, kCluThreads>;

@@ -240,10 +240,10 @@ struct LpRestartCopy {
     }
 };
 
-// A small LP's whole windows in one launch (cluster_windows.cuh), without the cuPDLPx ray
-// passes.
+// A small LP's whole windows in one launch (cluster_windows.cuh).
 template <typename TT>
 struct LpCluster : LpResident<TT> {
+    static constexpr bool kRays = false;
     using T = TT;
     using B = LpResident<TT>;
     using EvalCol = LpEvalColOp<T, kCluThreads>;
@@ -270,10 +270,43 @@ struct LpCluster : LpResident<TT> {
     __device__ const T* row_pdhg() const { return B::v.py; }
 };
 
+// The same with cuPDLPx termination: the ray passes (src/pdlp.jl:247-285) follow each full
+// evaluation.  Its own type, so that the plain windows' kernel carries none of it.
+// Four markshare-shaped LPs (6 x 56, 400-800 iterations): device 0.78-1.42 ms in one
+// block of lp_tiny_solve_kernel, 0.39-0.63 here.
+template <typename TT>
+struct LpClusterRays : LpCluster<TT> {
+    using T = TT;
+    using B = LpCluster<TT>;
+    static constexpr bool kRays = true;
+    using RayCol = RayColOp<kCluThreads>;
+    using RayRow = RayRowOp<kCluThreads>;
+    __device__ RayCol ray_col_op() const { return RayCol{B::d, B::st, nullptr, B::errp}; }
+    __device__ RayRow ray_row_op() const { return RayRow{B::d, B::st, B::errp}; }
+    __device__ void rays_begin() const {
+        if (threadIdx.x < 4) B::d.maxes[threadIdx.x] = 0ull;
+    }
+    __device__ void ray_col(int32_t j) const {
+        double none[2] = {0.0, 0.0};
+        RayRowsCol<T>{B::v, B::d, B::st}.row(j, 0, none);
+    }
+    __device__ double ray_row(int32_t i) const {
+        double slack[1] = {0.0};
+        RayRowsRow<T>{B::v, B::d, B::st, nullptr}.row(i, 0, slack);
+        return slack[0];
+    }
+    __device__ void rays_finalize(int p, const double* a) const {
+        LpRayFin{nullptr, nullptr, nullptr, nullptr, B::stw, B::d.maxes}.finalize(p, a);
+    }
+    __device__ void finalize(int p, const double* a, int32_t which) const {
+        LpController{nullptr, nullptr, nullptr, nullptr, B::stw, B::fl, which == EVAL_FULL ? 1 : 0, 1}.finalize(p, a);
+    }
+};
+
 // ---- a small LP's whole solve in one launch ---------------------------------------------
 //
-// With cuPDLPx termination, whose ray passes the cluster form lacks: one block runs whole evaluation
-// windows of pdlp_solve! (src/pdlp.jl:332-370) -- step 1, the evaluation after a
+// Where no cluster fits (cuPDLPx termination, or the FP64 polish of a mixed LP): one block
+// runs whole evaluation windows of pdlp_solve! (src/pdlp.jl:332-370) -- step 1, the evaluation after a
 // restart, steps 2 .. freq-1, step freq, the full evaluation, the cuPDLPx ray passes,
 // the controller and the restart copy -- until the LP stops, asks for the FP64 polish,
 // or max_windows windows have run.  STAGED: the LP's iterates, data, ray work vectors
@@ -474,9 +507,9 @@ class LpSolver {
             const char* te = std::getenv("PDFP_TINY");
             tiny_ = !(te && te[0] == '0') && static_cast<int64_t>(A.m) + A.n <= 4096 &&
                     M_.L.NNZ <= (1 << 16);
-            if (tiny_ && !cupdlpx_) {  // whole windows in a cluster, or else as a larger LP
-                if (f32_) clu32_.prepare<LpCluster<float>>(M_, ar_, max_smem_); else clu64_.prepare<LpCluster<double>>(M_, ar_, max_smem_);
-                tiny_ = (f32_ ? clu32_ : clu64_).ready();
+            if (tiny_) {  // whole windows in a cluster, or else as a larger LP (cuPDLPx: one block)
+                if (f32_) prepare_cluster<float>(); else prepare_cluster<double>();
+                tiny_ = cupdlpx_ || (f32_ ? clu32_ : clu64_).ready();
             }
         }
         m_ = A.m;
@@ -606,6 +639,8 @@ class LpSolver {
     template <typename T>
     void launch_tiny_solve();
     template <typename T>
+    ClusterForm& prepare_cluster();
+    template <typename T>
     void prepare_grids();
 
     bool cupdlpx_, f32_;
@@ -706,22 +741,33 @@ void LpSolver::record(int freq) {
     launch_elem(1, static_cast<int64_t>(n_) + m_, LpRestartCopy<T>{v, st_, n_, m_}, stream_);
 }
 
-// A small LP: up to kLpTinyWindowsPerLaunch windows in one launch (lp_tiny_solve_kernel).
+template <typename T>
+ClusterForm& LpSolver::prepare_cluster() {
+    ClusterForm& cf = std::is_same<T, float>::value ? clu32_ : clu64_;
+    if (cupdlpx_)
+        cf.template prepare<LpClusterRays<T>>(M_, ar_, max_smem_);
+    else
+        cf.template prepare<LpCluster<T>>(M_, ar_, max_smem_);
+    return cf;
+}
+
+// A small LP: many windows in one launch (cluster_windows.cuh, or lp_tiny_solve_kernel).
 template <typename T>
 void LpSolver::launch_tiny_solve() {
     LpVecs<T>* vp = nullptr;
     if constexpr (std::is_same<T, float>::value) vp = &v32_; else vp = &v64_;
-    ClusterForm& cf = std::is_same<T, float>::value ? clu32_ : clu64_;
-    if (!cupdlpx_) cf.template prepare<LpCluster<T>>(M_, ar_, max_smem_);
+    ClusterForm& cf = prepare_cluster<T>();
     if (cf.ready()) {
         cf.template fill<LpCluster<T>>(M_, ar_, stream_);
-        LpCluster<T> prob;
-        static_cast<LpResident<T>&>(prob) =
-            LpResident<T>{*vp, st_, std::is_same<T, float>::value ? MODE_FP32 : MODE_FP64, err_};
-        prob.d = d_;
-        prob.stw = st_;
-        prob.fl = flags_;
-        cf.launch(prob, M_, nullptr, stream_);
+        auto run = [&](auto prob) {
+            static_cast<LpResident<T>&>(prob) =
+                LpResident<T>{*vp, st_, std::is_same<T, float>::value ? MODE_FP32 : MODE_FP64, err_};
+            prob.d = d_;
+            prob.stw = st_;
+            prob.fl = flags_;
+            cf.launch(prob, M_, nullptr, stream_);
+        };
+        if (cupdlpx_) run(LpClusterRays<T>{}); else run(LpCluster<T>{});
         return;
     }
     const int32_t rowsum_len = 2 * std::max(std::max(n_, m_), 1);

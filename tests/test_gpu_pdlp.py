@@ -88,3 +88,33 @@ def test_small_lp_staged_equals_unstaged(monkeypatch, precision):
             out[stage] = (x, ds, status, iters)
         assert out["1"][2] == out["0"][2] and out["1"][3] == out["0"][3]
         assert np.array_equal(out["1"][0], out["0"][0]) and np.array_equal(out["1"][1], out["0"][1])
+
+
+def _ray_lp(case, m, n, seed):
+    """Sparse rows of four ones; infeasible: a row x_0 + x_1 <= -1 over x >= 0; unbounded: a last
+    column that only relaxes rows and pays."""
+    rng = np.random.default_rng(seed)
+    A = np.zeros((m, n))
+    for i in range(m):
+        A[i, rng.choice(n - 1, 4, replace=False)] = 1.0
+    b, c = np.full(m, 2.0), np.ones(n)
+    if case == "infeasible":
+        A[0] = 0.0
+        A[0, :2] = 1.0
+        b[0] = -1.0
+    else:
+        A[:, n - 1] = -1.0
+        c[n - 1] = -1.0
+    return _lp(A, b, c, np.zeros(n), np.full(n, np.inf), ["le"] * m)
+
+
+@pytest.mark.parametrize("m,n", [(5, 9), (33, 31), (300, 700), (900, 1500)])
+@pytest.mark.parametrize("case", ["infeasible", "unbounded"])
+def test_cupdlpx_rays_of_small_lps(oracle, case, m, n):
+    """The ray passes of small LPs, in one block and over a cluster's blocks: the status and the
+    iterations are the oracle's."""
+    milp = _ray_lp(case, m, n, 7)
+    _, _, so, io, _ = oracle.solve_lp_relaxation(milp, 1e-4, 30.0, True)
+    assert so == ("PRIMAL_INFEASIBLE" if case == "infeasible" else "DUAL_INFEASIBLE")
+    _, _, sg, ig = gpu.solve_lp_relaxation(milp, 1e-4, 30.0, True)
+    assert (sg, ig) == (so, io)
