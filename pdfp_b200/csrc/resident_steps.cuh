@@ -169,13 +169,14 @@ static __device__ __noinline__ bool res_gave_up(unsigned* dead, int32_t* err, ui
     return true;
 }
 
-// A piece of a long row, summed to `acc` by the lanes of a warp: the piece that arrives
-// last adds the row's pieces in order.  Returns the row (lane 0 of that warp; its sum in
-// acc), else -1.
+// A piece of a long row: the lanes' products pp[0], pp[32], .. (depth of them) and then the
+// lanes are summed in FP64, as in every engine's long rows; the piece that arrives last adds
+// the row's pieces in order.  Returns the row (lane 0 of that warp; its sum in acc), else -1.
 template <typename T>
 __device__ __noinline__ int32_t res_long(unsigned char* sm, const ResSide<T>& s, const ResSlice& m,
-                                         int32_t q, T& acc) {
-    double part = static_cast<double>(acc);
+                                         int32_t q, const T* pp, T& acc) {
+    double part = 0.0;
+    for (int u = 0; u < (m.shape >> 3); ++u) part += static_cast<double>(pp[32 * u]);
     for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
     if ((threadIdx.x & 31) != 0) return -1;
     const int32_t ln = reinterpret_cast<const int32_t*>(sm + s.lane)[q * 32];
@@ -326,11 +327,15 @@ __device__ __forceinline__ void res_pass(const P& prob, unsigned char* sm, const
             const ResPar<T>& pr = reinterpret_cast<const ResPar<T>*>(sm + s.par)[m.inst];
             p.weight = pr.weight[k & 1];  // written in the pass before
             p.omwt = pr.omwt[k & 1];
-            T acc = res_sum(prod + m.off + lane, m.shape >> 3);
+            const T* const pp = prod + m.off + lane;
+            T acc = T(0);
             if (piece) {
-                r = res_long<T>(sm, s, m, q, acc);
+                r = res_long<T>(sm, s, m, q, pp, acc);
                 if (r >= 0) read_vecs(r);
-            } else if (m.shape & 7) {
+            } else {
+                acc = res_sum(pp, m.shape >> 3);
+            }
+            if (!piece && (m.shape & 7)) {
                 const int G = 1 << (m.shape & 7);
 #pragma unroll 1
                 for (int o = G >> 1; o > 0; o >>= 1) acc = add_rn(acc, __shfl_xor_sync(0xffffffffu, acc, o));

@@ -225,3 +225,27 @@ def test_a_row_too_long_for_a_cluster_takes_the_resident_steps(oracle):
             h.solve(prm, 1.0)
         assert s.total_count == o.total_count
         assert np.linalg.norm(s.pdhg_x - o.pdhg_x) <= 1e-10 * max(1.0, np.linalg.norm(o.pdhg_x))
+
+
+@pytest.mark.gpu
+def test_long_rows_of_a_mixed_handle_are_summed_in_fp64(oracle, monkeypatch):
+    """One row of five pieces over columns fixed at 1: each lane's first entry is 1 and its
+    31 others 0.9 * 2^-24, which FP32 additions to 1 drop one by one (together 2.7e-4 of the
+    row's violation, all of it) and FP64 ones keep.  z, which grows by sigma times the
+    violation in every step, within 5% of the oracle's; products and x_bar carry at most
+    160 * 2 * 2^-24 = 1.9e-5 of rounding, 7% of the violation and of either sign."""
+    from pdfp_b200 import gpu
+    monkeypatch.setenv("PDFP_MIXED_MIN_NNZ", "0")
+    n = 5120
+    a = np.where(np.arange(n) % 1024 < 32, 1.0, 0.9 * 2.0 ** -24)
+    one = np.ones(n)
+    pr = (sp.csr_matrix(a[None, :]), np.array([160.0]), np.ones(1, np.uint8), np.zeros(n, np.uint8), one, one, one)
+    o = oracle.OracleSolvers.PDFPState(*pr)
+    prm = SolverParameters(eps_optimal_relative=1e-6, eps_feasible_relative=1e-6, iteration_limit=200)
+    s = _state(pr, "mixed", monkeypatch, "1")
+    for h in (s, o):
+        h.set_target(one)
+        h.set_x(one)
+        h.solve(prm, 1.0)
+    z, zo = s.get("pdhg_z")[0], o.get("pdhg_z")[0]
+    assert zo > 0.0 and abs(z - zo) <= 0.05 * zo
