@@ -21,7 +21,9 @@
 // Measured on one B200, FP64, whole solves, against one block that read the CSR arrays
 // from shared memory: that model, 600 iterations, 1.65 -> 0.58 ms; two 6 x 56 knapsacks
 // 1.11 -> 0.47; 601 x 1,503 with 15k nonzeros, 400 iterations, seven blocks, 8.6 -> 0.94;
-// the root LP of 133 x 201, whole call, 2.4 -> 1.27.
+// the root LP of 133 x 201, whole call, 2.4 -> 1.27.  Rows are whole whatever their length
+// (more than 512 entries: 32 lanes of more than 16): a 6 x 606 knapsack, 600 iterations,
+// 1.91 -> 1.00 ms, 2.43 with its rows in pieces on the resident window.
 //
 // A row's order of summation depends on its length alone and an evaluation's on the rows'
 // numbers alone, so the results do not depend on the cluster's size: a batch member takes
@@ -107,6 +109,8 @@ struct CluEntries {
     const uint32_t* ip;  // the entries after them
     const T* vp;
     int32_t depth;  // how many, a multiple of kCluDepthUnit
+    // A lane of more than kCluLaneNnz entries: one of 32 lanes of a row of more than 512.
+    __device__ __forceinline__ bool wide() const { return depth + kCluKept > kCluLaneNnz; }
     // zero: a shared address that holds 0
     __device__ __forceinline__ void take(const uint32_t* i, const T* v, int32_t d, uint32_t zero) {
 #pragma unroll
@@ -134,6 +138,14 @@ struct CluEntries {
 #pragma unroll
             for (int e = 0; e < kCluDepthUnit; ++e) acc = add_rn(acc, mul_rn(v[32 * e], y[e]));
         }
+        return acc;
+    }
+    // The same products, added in FP64: the lanes' sums of a wide row in the FP32 form.
+    __device__ __forceinline__ double sum64() const {
+        double acc = 0.0;
+#pragma unroll
+        for (int e = 0; e < kCluKept; ++e) acc += static_cast<double>(mul_rn(a[e], clu_load<T>(c[e])));
+        for (int e = 0; e < depth; ++e) acc += static_cast<double>(mul_rn(vp[32 * e], clu_load<T>(ip[32 * e])));
         return acc;
     }
 };
@@ -202,10 +214,18 @@ __device__ __forceinline__ void clu_steps(const P& prob, CluWarp<P>& w, const Cl
 #pragma unroll 1
     for (int32_t k = from; k < to; ++k) {
         if (ROW) cluster_meet<CL>();
-        T acc = w.entries.sum();
-        if (w.lanes > 1)
+        T acc;
+        if (sizeof(T) == 4 && w.entries.wide()) {  // the same for the whole warp
+            double sum = w.entries.sum64();
 #pragma unroll 1
-            for (int o = w.lanes >> 1; o > 0; o >>= 1) acc = add_rn(acc, __shfl_xor_sync(0xffffffffu, acc, o));
+            for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            acc = static_cast<T>(sum);
+        } else {
+            acc = w.entries.sum();
+            if (w.lanes > 1)
+#pragma unroll 1
+                for (int o = w.lanes >> 1; o > 0; o >>= 1) acc = add_rn(acc, __shfl_xor_sync(0xffffffffu, acc, o));
+        }
         if constexpr (ROW) {
             T in[P::NRV];
 #pragma unroll

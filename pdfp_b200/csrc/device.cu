@@ -291,9 +291,10 @@ bool DeviceMatrix::make_cluster(DeviceArena& ar, int c, int esize, int max_warps
                                 Resident& r, int& n_warps) const {
     r = Resident();
     HostResident ht, ha;
-    deal_resident(L.At, L.col_off, c, kCluLaneNnz, kCluDepthUnit, true, ht);
-    deal_resident(L.A, L.row_off, c, kCluLaneNnz, kCluDepthUnit, true, ha);
-    if (!ht.longs.empty() || !ha.longs.empty()) return false;
+    for (int p = 0; p < L.K; ++p) {  // every row whole: a lane sums a long row's every 32nd entry
+        deal_member(L.At, L.col_off, p, c, kCluLaneNnz, INT32_MAX, kCluDepthUnit, ht);
+        deal_member(L.A, L.row_off, p, c, kCluLaneNnz, INT32_MAX, kCluDepthUnit, ha);
+    }
     for (size_t b = 0; b < ht.blocks.size(); ++b) {
         const int p = static_cast<int>(b) / c;
         n_warps = std::max(b == 0 ? 1 : n_warps, ht.blocks[b].n_slices + ha.blocks[b].n_slices);

@@ -189,8 +189,8 @@ class DeviceMatrix {
     bool make_resident(DeviceArena& ar, int n_blocks, int esize, int ncv, int nrv, int par_bytes,
                        uint32_t max_smem, Resident& out) const;
     // The same for whole members in clusters of c blocks each (cluster_windows.cuh): false
-    // when a block would have more slices than warps, a row longer than a slice or more
-    // than max_smem bytes of shared memory; n_warps: the most slices of a block.
+    // when a block would have more slices than warps or more than max_smem bytes of shared
+    // memory; n_warps: the most slices of a block.
     bool make_cluster(DeviceArena& ar, int c, int esize, int max_warps, uint32_t max_smem, Resident& out,
                       int& n_warps) const;
     // The entries' values from this matrix's values of the same precision.

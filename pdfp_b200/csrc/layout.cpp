@@ -121,93 +121,127 @@ int32_t build_vec_items(const HostCsr& csr, const std::vector<int32_t>& inst_row
     return slots;
 }
 
-void deal_resident(const HostCsr& csr, const std::vector<int32_t>& inst_row_off, int n_blocks, int lane_nnz,
-                   int depth_unit, bool per_member, HostResident& o) {
-    o = HostResident();
+namespace {
+// Scratch of deal_block, kept over the blocks of a side.
+struct DealScratch {
+    std::vector<int32_t> order;
+    std::vector<ResSlice> sl;     // the block's slices
+    std::vector<int32_t> lr, by;  // their lanes' rows, their order
+};
+
+// The next block of a side: the packed rows [row0, row1), appended to o.  p: an instance at
+// or before row0's, advanced to it; a row of more than `piece` nonzeros is cut into pieces.
+void deal_block(const HostCsr& csr, const std::vector<int32_t>& inst_row_off, int32_t row0, int32_t row1,
+                int lane_nnz, int32_t piece, int depth_unit, int& p, DealScratch& w, HostResident& o) {
     const int K = static_cast<int>(inst_row_off.size()) - 1;
     const std::vector<int32_t>& rp = csr.rp;
-    const int32_t rows = csr.rows;
-    const double per_row = per_member ? 64.0 : 4.0;
-    const int32_t piece = 32 * lane_nnz;  // nonzeros per slice of a long row
     auto lanes_log2 = [&](int64_t len) {
         int lg = 0;
         while (lg < 5 && (int64_t(1) << lg) * lane_nnz < len) ++lg;
         return lg;
     };
-    int32_t r = 0;
-    int p = 0;
-    std::vector<int32_t> order;
-    std::vector<ResSlice> sl;   // one block's slices
-    std::vector<int32_t> lr, by;  // their lanes' rows, their order
-    for (int b = 0; b < (per_member ? K : 1) * n_blocks; ++b) {
-        // the rows [lo, hi) are dealt to n_blocks blocks, of which this is number `nth`
-        const int32_t lo = per_member ? inst_row_off[b / n_blocks] : 0;
-        const int32_t hi = per_member ? inst_row_off[b / n_blocks + 1] : rows;
-        const int nth = b % n_blocks;
-        ResBlock B{};
-        B.row0 = r;
-        const double want = hi > lo ? (static_cast<double>(rp[hi]) - rp[lo] + per_row * (hi - lo)) * (nth + 1) / n_blocks : 0.0;
-        while (r < hi && (nth + 1 == n_blocks ||
-                          static_cast<double>(rp[r + 1]) - rp[lo] + per_row * (r + 1 - lo) <= want + 0.5)) ++r;
-        B.row1 = r;
-        B.slice0 = static_cast<int32_t>(o.slices.size());
-        B.elem0 = b > 0 ? o.blocks.back().elem0 + o.blocks.back().n_elem : 0;
-        B.long0 = static_cast<int32_t>(o.longs.size());
-        while (p + 1 < K && inst_row_off[p + 1] <= B.row0) ++p;
-        B.inst0 = p;
-        sl.clear();
-        lr.clear();
-        auto add_slice = [&](int depth, int lg, int inst, int slot, int32_t row) {
-            depth = (depth + depth_unit - 1) / depth_unit * depth_unit;
-            sl.push_back(ResSlice{B.n_elem, depth * 8 + lg, inst, slot});
-            lr.resize(lr.size() + 32, row);
-            B.n_elem += 32 * depth;
-        };
-        int q = p;
-        for (int32_t a = B.row0; a < B.row1;) {  // one instance's rows at a time
-            while (q + 1 < K && inst_row_off[q + 1] <= a) ++q;
-            const int32_t e = std::min(B.row1, inst_row_off[q + 1]);
-            order.resize(e - a);
-            std::iota(order.begin(), order.end(), a);
-            auto longer = [&](int32_t x, int32_t y) { return rp[x + 1] - rp[x] > rp[y + 1] - rp[y]; };
-            if (!std::is_sorted(order.begin(), order.end(), longer))
-                std::stable_sort(order.begin(), order.end(), longer);
-            for (size_t i = 0; i < order.size();) {
-                const int32_t row = order[i], len = rp[row + 1] - rp[row];
-                if (len > piece) {
-                    const int32_t np = (len + piece - 1) / piece;
-                    o.longs.push_back(ResLong{row - B.row0, B.n_slots, np, q - B.inst0});
-                    for (int32_t s = 0; s < np; ++s)
-                        add_slice((std::min(piece, len - s * piece) + 31) / 32, 5, q - B.inst0,
-                                  B.n_slots++, static_cast<int32_t>(o.longs.size()) - 1 - B.long0);
-                    ++i;
-                    continue;
-                }
-                const int lg = lanes_log2(len), G = 1 << lg, per = 32 >> lg;
-                const size_t lane0 = lr.size();
-                add_slice((len + G - 1) / G, lg, q - B.inst0, -1, -1);  // the longest row comes first
-                for (int g = 0; g < per && i < order.size(); ++g, ++i) {
-                    if (lanes_log2(rp[order[i] + 1] - rp[order[i]]) != lg) break;
-                    std::fill_n(lr.begin() + lane0 + g * G, G, order[i] - B.row0);
-                }
+    std::vector<int32_t>& order = w.order;
+    std::vector<ResSlice>& sl = w.sl;
+    std::vector<int32_t>&lr = w.lr, &by = w.by;
+    ResBlock B{};
+    B.row0 = row0;
+    B.row1 = row1;
+    B.slice0 = static_cast<int32_t>(o.slices.size());
+    B.elem0 = o.blocks.empty() ? 0 : o.blocks.back().elem0 + o.blocks.back().n_elem;
+    B.long0 = static_cast<int32_t>(o.longs.size());
+    while (p + 1 < K && inst_row_off[p + 1] <= B.row0) ++p;
+    B.inst0 = p;
+    sl.clear();
+    lr.clear();
+    auto add_slice = [&](int depth, int lg, int inst, int slot, int32_t row) {
+        depth = (depth + depth_unit - 1) / depth_unit * depth_unit;
+        sl.push_back(ResSlice{B.n_elem, depth * 8 + lg, inst, slot});
+        lr.resize(lr.size() + 32, row);
+        B.n_elem += 32 * depth;
+    };
+    int q = p;
+    for (int32_t a = B.row0; a < B.row1;) {  // one instance's rows at a time
+        while (q + 1 < K && inst_row_off[q + 1] <= a) ++q;
+        const int32_t e = std::min(B.row1, inst_row_off[q + 1]);
+        order.resize(e - a);
+        std::iota(order.begin(), order.end(), a);
+        auto longer = [&](int32_t x, int32_t y) { return rp[x + 1] - rp[x] > rp[y + 1] - rp[y]; };
+        if (!std::is_sorted(order.begin(), order.end(), longer))
+            std::stable_sort(order.begin(), order.end(), longer);
+        for (size_t i = 0; i < order.size();) {
+            const int32_t row = order[i], len = rp[row + 1] - rp[row];
+            if (len > piece) {
+                const int32_t np = (len + piece - 1) / piece;
+                o.longs.push_back(ResLong{row - B.row0, B.n_slots, np, q - B.inst0});
+                for (int32_t s = 0; s < np; ++s)
+                    add_slice((std::min(piece, len - s * piece) + 31) / 32, 5, q - B.inst0,
+                              B.n_slots++, static_cast<int32_t>(o.longs.size()) - 1 - B.long0);
+                ++i;
+                continue;
             }
-            a = e;
+            const int lg = lanes_log2(len), G = 1 << lg, per = 32 >> lg;
+            const size_t lane0 = lr.size();
+            add_slice((len + G - 1) / G, lg, q - B.inst0, -1, -1);  // the longest row comes first
+            for (int g = 0; g < per && i < order.size(); ++g, ++i) {
+                if (lanes_log2(rp[order[i] + 1] - rp[order[i]]) != lg) break;
+                std::fill_n(lr.begin() + lane0 + g * G, G, order[i] - B.row0);
+            }
         }
-        B.n_inst = B.row1 > B.row0 ? q - B.inst0 + 1 : 0;
-        B.n_slices = static_cast<int32_t>(sl.size());
-        B.n_long = static_cast<int32_t>(o.longs.size()) - B.long0;
-        // deepest slices first, so that the warps' last rounds are the short ones
-        by.resize(sl.size());
-        std::iota(by.begin(), by.end(), 0);
-        std::stable_sort(by.begin(), by.end(), [&](int32_t x, int32_t y) {
-            return (sl[x].shape >> 3) > (sl[y].shape >> 3);
-        });
-        for (int32_t s : by) {
-            o.slices.push_back(sl[s]);
-            o.lane_row.insert(o.lane_row.end(), lr.begin() + size_t(32) * s, lr.begin() + size_t(32) * (s + 1));
-        }
-        o.blocks.push_back(B);
+        a = e;
     }
+    B.n_inst = B.row1 > B.row0 ? q - B.inst0 + 1 : 0;
+    B.n_slices = static_cast<int32_t>(sl.size());
+    B.n_long = static_cast<int32_t>(o.longs.size()) - B.long0;
+    // deepest slices first, so that the warps' last rounds are the short ones
+    by.resize(sl.size());
+    std::iota(by.begin(), by.end(), 0);
+    std::stable_sort(by.begin(), by.end(), [&](int32_t x, int32_t y) {
+        return (sl[x].shape >> 3) > (sl[y].shape >> 3);
+    });
+    for (int32_t s : by) {
+        o.slices.push_back(sl[s]);
+        o.lane_row.insert(o.lane_row.end(), lr.begin() + size_t(32) * s, lr.begin() + size_t(32) * (s + 1));
+    }
+    o.blocks.push_back(B);
+}
+
+// The rows [lo, hi) to n_blocks blocks of about equal nonzeros + per_row per row.
+void deal_range(const HostCsr& csr, const std::vector<int32_t>& inst_row_off, int32_t lo, int32_t hi, int n_blocks,
+                double per_row, int lane_nnz, int32_t piece, int depth_unit, int& p, DealScratch& w,
+                HostResident& o) {
+    const std::vector<int32_t>& rp = csr.rp;
+    int32_t r = lo;
+    for (int b = 0; b < n_blocks; ++b) {
+        const int32_t row0 = r;
+        const double want =
+            hi > lo ? (static_cast<double>(rp[hi]) - rp[lo] + per_row * (hi - lo)) * (b + 1) / n_blocks : 0.0;
+        while (r < hi && (b + 1 == n_blocks ||
+                          static_cast<double>(rp[r + 1]) - rp[lo] + per_row * (r + 1 - lo) <= want + 0.5)) ++r;
+        deal_block(csr, inst_row_off, row0, r, lane_nnz, piece, depth_unit, p, w, o);
+    }
+}
+}  // namespace
+
+void deal_member(const HostCsr& csr, const std::vector<int32_t>& inst_row_off, int member, int n_blocks,
+                 int lane_nnz, int32_t piece, int depth_unit, HostResident& o) {
+    DealScratch w;
+    int p = member;
+    deal_range(csr, inst_row_off, inst_row_off[member], inst_row_off[member + 1], n_blocks, 64.0, lane_nnz, piece,
+               depth_unit, p, w, o);
+}
+
+void deal_resident(const HostCsr& csr, const std::vector<int32_t>& inst_row_off, int n_blocks, int lane_nnz,
+                   int depth_unit, bool per_member, HostResident& o) {
+    o = HostResident();
+    const int K = static_cast<int>(inst_row_off.size()) - 1;
+    if (per_member) {
+        for (int p = 0; p < K; ++p)
+            deal_member(csr, inst_row_off, p, n_blocks, lane_nnz, 32 * lane_nnz, depth_unit, o);
+        return;
+    }
+    DealScratch w;
+    int p = 0;
+    deal_range(csr, inst_row_off, 0, csr.rows, n_blocks, 4.0, lane_nnz, 32 * lane_nnz, depth_unit, p, w, o);
 }
 
 void fill_resident(const HostCsr& csr, int lane_nnz, HostResident& o) {

@@ -269,6 +269,10 @@ struct HostResident {
 // Slice depths are rounded up to a multiple of depth_unit.
 void deal_resident(const HostCsr& csr, const std::vector<int32_t>& inst_row_off, int n_blocks, int lane_nnz,
                    int depth_unit, bool per_member, HostResident& out);
+// One member's rows to n_blocks blocks, appended to `out` (deal_resident's per_member form,
+// in which `piece` is 32 * lane_nnz): rows of up to `piece` nonzeros stay whole.
+void deal_member(const HostCsr& csr, const std::vector<int32_t>& inst_row_off, int member, int n_blocks,
+                 int lane_nnz, int32_t piece, int depth_unit, HostResident& out);
 void fill_resident(const HostCsr& csr, int lane_nnz, HostResident& out);
 // Dynamic shared memory a block needs for its share of both sides, with `esize`-byte
 // reals, ncv / nrv vectors kept per column / row and par_bytes of parameters per

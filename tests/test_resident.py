@@ -249,3 +249,46 @@ def test_long_rows_of_a_mixed_handle_are_summed_in_fp64(oracle, monkeypatch):
         h.solve(prm, 1.0)
     z, zo = s.get("pdhg_z")[0], o.get("pdhg_z")[0]
     assert zo > 0.0 and abs(z - zo) <= 0.05 * zo
+
+
+def _wide(seed, m, n, row_len):
+    """Few rows of row_len nonzeros over binary columns, one of them an equality."""
+    rng = np.random.default_rng(seed)
+    A = sp.lil_matrix((m, n))
+    for i in range(m):
+        A[i, np.sort(rng.choice(n, size=row_len, replace=False))] = rng.uniform(0.5, 2.0, size=row_len)
+    A = sp.csr_matrix(A)
+    A.sort_indices()
+    b = 0.5 * (A @ np.ones(n))
+    eq = np.zeros(m, np.uint8)
+    eq[0] = 1
+    sc = 1.0 / np.sqrt(row_len)
+    return (A * sc, b * sc, eq, np.ones(n, np.uint8), np.zeros(n), np.ones(n), np.ones(n)), np.round(rng.random(n))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("m,n,row_len,window_form", [(3, 520, 512, 3), (3, 520, 513, 3), (6, 606, 601, 3),
+                                                     (5, 1300, 1025, 3), (3, 3500, 3300, 3), (4, 4092, 4000, 4)])
+def test_wide_rows_run_in_a_cluster(oracle, monkeypatch, precision, m, n, row_len, window_form):
+    """A small member with rows of any length runs its windows in a cluster (lanes deeper than
+    their usual 16 entries), unless it has more slices (128 of 32 columns and 4 rows) than
+    eight blocks have warps; to the bounds of the resident steps' test: 1e-10 of the oracle,
+    2e-4 in FP32."""
+    from pdfp_b200 import gpu
+    monkeypatch.setenv("PDFP_MIXED_MIN_NNZ", "0")
+    pr, xt = _wide(9, m, n, row_len)
+    tol = 1e-10 if precision == "fp64" else 2e-4
+    for windows in (1, 3):
+        prm = SolverParameters(eps_optimal_relative=1e-6, eps_feasible_relative=1e-6, iteration_limit=200 * windows)
+        s, o = gpu.PDFPState(*pr, precision=precision), oracle.OracleSolvers.PDFPState(*pr)
+        form = gpu.C.c_int32()
+        gpu.L.check(gpu.L.lib().pdfp_get_window_form(s._h, gpu.C.byref(form)))
+        assert form.value == window_form
+        for h in (s, o):
+            h.set_target(xt)
+            h.solve(prm, 1.0)
+        assert s.total_count == o.total_count
+        for name in ("pdhg_x", "pdhg_y", "pdhg_z", "current_x", "current_y", "current_z"):
+            a, b = s.get(name), o.get(name)
+            assert np.linalg.norm(a - b) <= tol * max(1.0, np.linalg.norm(b)), (windows, name)
