@@ -287,23 +287,59 @@ bool DeviceMatrix::make_resident(DeviceArena& ar, int n_blocks, int esize, int n
     return true;
 }
 
-bool DeviceMatrix::make_cluster(DeviceArena& ar, int c, int esize, int max_warps, uint32_t max_smem,
-                                Resident& r, int& n_warps) const {
+bool DeviceMatrix::make_cluster(DeviceArena& ar, int max_blocks, int esize, int max_warps, uint32_t max_smem,
+                                Resident& r, std::vector<ClusterGroup>& groups) const {
     r = Resident();
+    groups.clear();
     HostResident ht, ha;
-    for (int p = 0; p < L.K; ++p) {  // every row whole: a lane sums a long row's every 32nd entry
-        deal_member(L.At, L.col_off, p, c, kCluLaneNnz, INT32_MAX, kCluDepthUnit, ht);
-        deal_member(L.A, L.row_off, p, c, kCluLaneNnz, INT32_MAX, kCluDepthUnit, ha);
+    std::vector<ClusterGroup> by(max_blocks + 1);
+    std::vector<std::vector<ClusterMember>> in(max_blocks + 1);
+    for (int p = 0; p < L.K; ++p) {
+        const int32_t n = L.col_off[p + 1] - L.col_off[p], m = L.row_off[p + 1] - L.row_off[p];
+        const int32_t b0 = static_cast<int32_t>(ht.blocks.size());
+        int warps = 0;
+        uint32_t smem = 0;
+        // the fewest blocks that hold the member, every row whole: a lane sums a long
+        // row's every 32nd entry
+        auto fits = [&](int c) {
+            for (HostResident* o : {&ht, &ha}) {  // without the blocks of the number tried before
+                if (static_cast<int32_t>(o->blocks.size()) == b0) continue;
+                o->slices.resize(o->blocks[b0].slice0);
+                o->lane_row.resize(size_t(32) * o->slices.size());
+                o->blocks.resize(b0);
+            }
+            deal_member(L.At, L.col_off, p, c, kCluLaneNnz, INT32_MAX, kCluDepthUnit, ht);
+            deal_member(L.A, L.row_off, p, c, kCluLaneNnz, INT32_MAX, kCluDepthUnit, ha);
+            warps = 1;
+            smem = 0;
+            for (int b = b0; b < b0 + c; ++b) {
+                warps = std::max(warps, ht.blocks[b].n_slices + ha.blocks[b].n_slices);
+                smem = std::max(smem, clu_smem(ht.blocks[b], ha.blocks[b], esize, n, m).total);
+            }
+            return warps <= max_warps && smem <= max_smem;
+        };
+        int c = 1;
+        if (!fits(1)) {  // more blocks never make fewer slices
+            c = std::max(2, (warps + max_warps - 1) / max_warps);
+            while (c <= max_blocks && !fits(c)) ++c;
+            if (c > max_blocks) return false;
+        }
+        by[c].n_warps = std::max(by[c].n_warps, warps);
+        by[c].smem = std::max(by[c].smem, smem);
+        in[c].push_back(ClusterMember{p, b0});
     }
-    for (size_t b = 0; b < ht.blocks.size(); ++b) {
-        const int p = static_cast<int>(b) / c;
-        n_warps = std::max(b == 0 ? 1 : n_warps, ht.blocks[b].n_slices + ha.blocks[b].n_slices);
-        if (n_warps > max_warps) return false;
-        r.smem = std::max(r.smem, clu_smem(ht.blocks[b], ha.blocks[b], esize, L.col_off[p + 1] - L.col_off[p],
-                                           L.row_off[p + 1] - L.row_off[p]).total);
+    std::vector<ClusterMember> all;
+    for (int c = max_blocks; c >= 1; --c) {  // the largest members first
+        if (in[c].empty()) continue;
+        by[c].n_ranks = c;
+        by[c].first = static_cast<int32_t>(all.size());
+        by[c].count = static_cast<int32_t>(in[c].size());
+        groups.push_back(by[c]);
+        all.insert(all.end(), in[c].begin(), in[c].end());
     }
-    if (r.smem > max_smem) return false;
     upload_resident(ar, ht, ha, kCluLaneNnz, r);
+    const ClusterMember* d = ar.upload(all);
+    for (ClusterGroup& g : groups) g.members = d + g.first;
     return true;
 }
 

@@ -188,11 +188,19 @@ class DeviceMatrix {
     };
     bool make_resident(DeviceArena& ar, int n_blocks, int esize, int ncv, int nrv, int par_bytes,
                        uint32_t max_smem, Resident& out) const;
-    // The same for whole members in clusters of c blocks each (cluster_windows.cuh): false
-    // when a block would have more slices than warps or more than max_smem bytes of shared
-    // memory; n_warps: the most slices of a block.
-    bool make_cluster(DeviceArena& ar, int c, int esize, int max_warps, uint32_t max_smem, Resident& out,
-                      int& n_warps) const;
+    // The same for whole members in clusters (cluster_windows.cuh), each of as few blocks as
+    // hold it, up to max_blocks: false when a member's blocks would need more than max_warps
+    // slices or max_smem bytes of shared memory.  The members of one number of blocks form a
+    // group, the largest number first.
+    struct ClusterGroup {
+        int n_ranks = 0;     // blocks per member
+        int n_warps = 1;     // the most slices of a block
+        uint32_t smem = 0;   // dynamic shared memory of the largest block
+        int32_t first = 0, count = 0;
+        const ClusterMember* members = nullptr;  // device: its members
+    };
+    bool make_cluster(DeviceArena& ar, int max_blocks, int esize, int max_warps, uint32_t max_smem, Resident& out,
+                      std::vector<ClusterGroup>& groups) const;
     // The entries' values from this matrix's values of the same precision.
     void fill_resident(DeviceArena& ar, Resident& r, bool f32, cudaStream_t s) const;
   private:

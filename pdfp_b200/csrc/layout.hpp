@@ -343,6 +343,11 @@ PDFP_HD inline CluSmem clu_smem(const ResBlock& t, const ResBlock& a, int esize,
     return s;
 }
 
+// A member of a cluster launch and the first of its blocks.
+struct ClusterMember {
+    int32_t inst, block0;
+};
+
 // Device view of one side.
 struct ResDev {
     const ResBlock* blocks = nullptr;

@@ -292,3 +292,41 @@ def test_wide_rows_run_in_a_cluster(oracle, monkeypatch, precision, m, n, row_le
         for name in ("pdhg_x", "pdhg_y", "pdhg_z", "current_x", "current_y", "current_z"):
             a, b = s.get(name), o.get(name)
             assert np.linalg.norm(a - b) <= tol * max(1.0, np.linalg.norm(b)), (windows, name)
+
+
+@pytest.mark.gpu
+def test_members_of_several_sizes_in_clusters_of_their_own(oracle):
+    """400 members of one block each beside one of seven: the device time of the batch is at
+    most twice that of its parts one after the other (a cluster of seven blocks for every
+    member takes eight times the part of the 400), and the members' results are their own
+    handles', bit for bit."""
+    from pdfp_b200 import gpu
+    small = synthetic.covering_p0201_like(1)
+    big = synthetic.general_integer(6, m=601, n=1503, m_eq=150, mean_row=25.0)[0]
+    inputs = {}
+    for m in (small, big):
+        sc, is_eq, is_int, w = oracle.projector_inputs(m)
+        inputs[id(m)] = (sc.A, sc.con_ub, is_eq, is_int, sc.var_lb, sc.var_ub, w)
+    prm = SolverParameters(eps_optimal_relative=1e-9, eps_feasible_relative=1e-9, iteration_limit=400)
+
+    def solved(models):
+        b = gpu.PDFPBatch([inputs[id(m)] for m in models], precision="fp64")
+        for _ in range(2):  # the second solve is timed
+            for p, m in enumerate(models):
+                rng = np.random.default_rng(p % 5)
+                b.set_target(p, np.round(rng.random(len(m.c))))
+            b.solve(prm, 1.0)
+        return b
+
+    many = [small] * 400
+    both = solved(many[:200] + [big] + many[200:])
+    parts = [solved(many), solved([big])]
+    assert both.results[0]["device_ms"] <= 2.0 * sum(b.results[0]["device_ms"] for b in parts)
+    for p in (0, 3, 199, 200, 201, 400):
+        m = big if p == 200 else small
+        s = gpu.PDFPState(*inputs[id(m)], precision="fp64")
+        for _ in range(2):
+            s.set_target(np.round(np.random.default_rng(p % 5).random(len(m.c))))
+            s.solve(prm, 1.0)
+        for name in ("pdhg_x", "pdhg_z", "current_y"):
+            assert np.array_equal(s.get(name), both.get(p, name)), (p, name)
