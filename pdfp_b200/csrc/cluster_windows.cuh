@@ -310,7 +310,9 @@ __device__ __forceinline__ void clu_eval(const Op& op, const int32_t* rp, const 
 }
 
 // Windows of members[blockIdx.x / n_ranks].  P: the steps (as the resident window's), the
-// evaluation Ops and the controller.
+// evaluation Ops and the controller.  any_stop: a member that stops sets it, and the others
+// leave after their window; each runs one at least, also where more members than the GPU
+// holds clusters at a time wait for the first ones to leave (of eight blocks, 16 or so).
 template <class P, bool CL>
 __global__ void __launch_bounds__(kCluThreads, 1)
     cluster_windows_kernel(const P prob, const ResDev dt, const ResDev da, const int32_t* rp_t,
@@ -362,14 +364,6 @@ __global__ void __launch_bounds__(kCluThreads, 1)
     if (is_row) w = clu_warp<true, P>(prob, sm, da, ba, warp - bt.n_slices, o.idx_a, o.val_a, o.zs, r0, xs + n);
     const bool eq = is_row && w.i >= 0 && w.i < prob.eq_end(p);
     cluster_meet<CL>();
-    if (any_stop) {  // another member may have stopped: the first block's answer holds for all
-        if (rank == 0 && threadIdx.x == 0) {
-            const int32_t go = ctl.go && !*reinterpret_cast<volatile int32_t*>(any_stop);
-            for (uint32_t b = 0; b < n_ranks; ++b)
-                cluster_put(CL ? cluster_map(smem_addr(&ctl.go), b) : smem_addr(&ctl.go), go);
-        }
-        cluster_meet<CL>();
-    }
     auto minor = [&](int32_t from, int32_t to) {
         if (is_col) {
             clu_steps<false, false, CL>(prob, w, ctl, false, from, to, n_ranks);

@@ -87,3 +87,25 @@ def test_resume_needs_a_running_member(oracle, examples):
     b.warm_start(1)  # a new projection for member 1: it can no longer resume
     with pytest.raises(Exception, match="cannot resume"):
         b.solve_any([IDLE, TIGHT], 1.0, resume=[False, True])
+
+
+def test_members_that_wait_for_a_cluster_advance_too(oracle):
+    """64 members of seven blocks each, of which the GPU holds about 16 at a time: the first
+    one stops after one window, and when the call returns every other one has run a window at
+    least, as its own handle would."""
+    milp, _, xt = synthetic.general_integer(6, m=601, n=1503, m_eq=150, mean_row=25.0)
+    sc, is_eq, is_int, w = oracle.projector_inputs(milp)
+    pr = (sc.A, sc.con_ub, is_eq, is_int, sc.var_lb, sc.var_ub, w)
+    K = 64
+    b = gpu.PDFPBatch([pr] * K, precision="fp64")
+    for p in range(K):
+        b.set_target(p, xt / sc.D_c)
+    never = dict(eps_optimal_relative=1e-12, eps_feasible_relative=1e-12)
+    st = b.solve_any([SolverParameters(iteration_limit=200 if p == 0 else 10 ** 6, **never) for p in range(K)], 1.0)
+    assert st[0] == "ITERATION_LIMIT" and st[1:] == ["RUNNING"] * (K - 1)
+    totals = [r["total_count"] for r in b.results]
+    assert min(totals) >= 200
+    s = gpu.PDFPState(*pr)
+    s.set_target(xt / sc.D_c)
+    s.solve(SolverParameters(iteration_limit=totals[K - 1], **never), 1.0)
+    assert np.array_equal(s.pdhg_x, b.get(K - 1, "pdhg_x"))
