@@ -259,9 +259,8 @@ bool DeviceMatrix::make_seg(DeviceArena& ar, int nseg, int long_min, const Stage
 constexpr int32_t kResHotRow = 512;
 constexpr int64_t kResHotNnz = int64_t(1) << 18;
 
-bool DeviceMatrix::make_resident(DeviceArena& ar, int n_blocks, int esize, int ncv, int nrv,
-                                 int par_bytes, uint32_t max_smem, Resident& r) const {
-    r = Resident();
+bool DeviceMatrix::plan_resident(int n_blocks, int esize, int ncv, int nrv, int par_bytes, uint32_t max_smem,
+                                 HostResident& ht, HostResident& ha, uint32_t& smem) const {
     // entries and vectors alone, spread evenly: no need to lay out what cannot fit
     const double least = 2.0 * L.NNZ * (4 + 2 * esize) +
                          static_cast<double>(esize * ncv + 4) * L.N + static_cast<double>(esize * nrv + 4) * L.M;
@@ -277,14 +276,12 @@ bool DeviceMatrix::make_resident(DeviceArena& ar, int n_blocks, int esize, int n
                 if (s->rp[i + 1] - s->rp[i] >= kResHotRow) hot += s->rp[i + 1] - s->rp[i];
         if (2 * hot > L.NNZ) return false;
     }
-    HostResident ht, ha;
     deal_resident(L.At, L.col_off, n_blocks, kResLaneNnz, 1, false, ht);
     deal_resident(L.A, L.row_off, n_blocks, kResLaneNnz, 1, false, ha);
+    smem = 0;
     for (int b = 0; b < n_blocks; ++b)
-        r.smem = std::max(r.smem, res_smem(ht.blocks[b], ha.blocks[b], esize, ncv, nrv, par_bytes).total);
-    if (r.smem > max_smem) return false;
-    upload_resident(ar, ht, ha, kResLaneNnz, r);
-    return true;
+        smem = std::max(smem, res_smem(ht.blocks[b], ha.blocks[b], esize, ncv, nrv, par_bytes).total);
+    return smem <= max_smem;
 }
 
 bool DeviceMatrix::make_cluster(DeviceArena& ar, int max_blocks, int esize, int max_warps, uint32_t max_smem,
@@ -337,60 +334,90 @@ bool DeviceMatrix::make_cluster(DeviceArena& ar, int max_blocks, int esize, int 
         groups.push_back(by[c]);
         all.insert(all.end(), in[c].begin(), in[c].end());
     }
-    upload_resident(ar, ht, ha, kCluLaneNnz, r);
+    upload_resident(ar, ht, ha, INT32_MAX, r);
     const ClusterMember* d = ar.upload(all);
     for (ClusterGroup& g : groups) g.members = d + g.first;
     return true;
 }
 
-void DeviceMatrix::upload_resident(DeviceArena& ar, HostResident& ht, HostResident& ha, int lane_nnz,
+void DeviceMatrix::upload_resident(DeviceArena& ar, const HostResident& ht, const HostResident& ha, int32_t piece,
                                    Resident& r) const {
-    ::pdfp::fill_resident(L.At, lane_nnz, ht);
-    ::pdfp::fill_resident(L.A, lane_nnz, ha);
-    const std::vector<void*> d = ar.upload_group(
-        {part(ht.blocks), part(ht.slices), part(ht.longs), part(ht.lane_row), part(ht.idx), part(ht.src),
-         part(ha.blocks), part(ha.slices), part(ha.longs), part(ha.lane_row), part(ha.idx), part(ha.src)});
+    const std::vector<void*> d = ar.upload_group({part(ht.blocks), part(ht.slices), part(ht.longs), part(ht.lane_row),
+                                                  part(ha.blocks), part(ha.slices), part(ha.longs), part(ha.lane_row)});
     auto side = [&](int k) {
         ResDev s;
         s.blocks = static_cast<const ResBlock*>(d[k]);
         s.slices = static_cast<const ResSlice*>(d[k + 1]);
         s.longs = static_cast<const ResLong*>(d[k + 2]);
         s.lane_row = static_cast<const int32_t*>(d[k + 3]);
-        s.idx = static_cast<const int32_t*>(d[k + 4]);
         return s;
     };
+    auto entries = [](const HostResident& h) {
+        return h.blocks.empty() ? int64_t(0) : int64_t(h.blocks.back().elem0) + h.blocks.back().n_elem;
+    };
     r.t = side(0);
-    r.a = side(6);
-    r.src_t = static_cast<const int32_t*>(d[5]);
-    r.src_a = static_cast<const int32_t*>(d[11]);
-    r.n_t = static_cast<int64_t>(ht.src.size());
-    r.n_a = static_cast<int64_t>(ha.src.size());
+    r.a = side(4);
+    r.n_t = entries(ht);
+    r.n_a = entries(ha);
+    r.piece = piece;
     r.n_blocks = static_cast<int>(ht.blocks.size());
     // the copies from pageable memory may still be under way on the default stream, which
     // the handle's own stream does not wait for
     PDFP_CK(cudaStreamSynchronize(0));
 }
 
+// The entries of a layout in slices, one warp per slice: fill_resident() of layout.cpp, which
+// states what goes where, on the arrays of the CSR matrix.  A new handle's first solve of one
+// window, in per-step launches / resident with this / with the entries made by a host thread
+// and uploaded: FP64 600k nonzeros 9.4 / 8.5 / 12.2 ms, mixed 900k 16.0 / 15.0 / 20.4.
 template <typename T>
-__global__ void gather_values_kernel(const int32_t* __restrict__ src, const T* __restrict__ val,
-                                     T* __restrict__ out, int64_t n) {
-    for (int64_t i = blockIdx.x * int64_t(256) + threadIdx.x; i < n; i += int64_t(gridDim.x) * 256)
-        out[i] = src[i] >= 0 ? val[src[i]] : T(0);
+__global__ void __launch_bounds__(256) fill_slices_kernel(const ResDev d, int n_blocks, int32_t piece,
+                                                          const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
+                                                          const T* __restrict__ v, int32_t* __restrict__ idx,
+                                                          T* __restrict__ val) {
+    const int lane = threadIdx.x & 31;
+    for (int b = blockIdx.x; b < n_blocks; b += gridDim.x) {
+        const ResBlock B = d.blocks[b];
+        for (int32_t q = blockIdx.y * 8 + (threadIdx.x >> 5); q < B.n_slices; q += gridDim.y * 8) {
+            const ResSlice m = d.slices[B.slice0 + q];
+            const int lg = m.shape & 7;
+            const int32_t ln = d.lane_row[int64_t(32) * (B.slice0 + q) + lane];
+            int32_t k = 0, end = 0;  // the lane's entries: every 2^lg-th of its row or piece
+            if (ln >= 0) {
+                const ResLong l = m.slot >= 0 ? d.longs[B.long0 + ln] : ResLong{};
+                const int32_t row = B.row0 + (m.slot >= 0 ? l.row : ln);
+                const int32_t k0 = rp[row] + (m.slot >= 0 ? (m.slot - l.slot0) * piece : 0);
+                end = m.slot >= 0 && rp[row + 1] - k0 > piece ? k0 + piece : rp[row + 1];
+                k = k0 + (lane & ((1 << lg) - 1));
+            }
+            int64_t x = int64_t(B.elem0) + m.off + lane;
+            for (int u = 0; u < (m.shape >> 3); ++u, x += 32, k += 1 << lg) {
+                idx[x] = k < end ? ci[k] : -1;
+                val[x] = k < end ? v[k] : T(0);
+            }
+        }
+    }
 }
 
 template <typename T>
-static const void* resident_values(DeviceArena& ar, const int32_t* src, const T* val, int64_t n,
-                                   cudaStream_t s) {
-    T* out = ar.alloc<T>(n);
-    const int blocks = static_cast<int>(std::min<int64_t>((n + 255) / 256, 4096));
-    if (n > 0) gather_values_kernel<T><<<blocks, 256, 0, s>>>(src, val, out, n);
+static void fill_slices(DeviceArena& ar, ResDev& d, int64_t n, int n_blocks, int32_t piece, const int32_t* rp,
+                        const int32_t* ci, const T* v, cudaStream_t s) {
+    int32_t* const idx = ar.alloc<int32_t>(n);
+    T* const val = ar.alloc<T>(n);
+    fill_slices_kernel<T><<<dim3(std::min(n_blocks, 4096), 8), 256, 0, s>>>(d, n_blocks, piece, rp, ci, v, idx, val);
     PDFP_CK(cudaGetLastError());
-    return out;
+    d.idx = idx;
+    d.val = val;
 }
 
 void DeviceMatrix::fill_resident(DeviceArena& ar, Resident& r, bool f32, cudaStream_t s) const {
-    r.t.val = f32 ? resident_values(ar, r.src_t, v32_t, r.n_t, s) : resident_values(ar, r.src_t, v64_t, r.n_t, s);
-    r.a.val = f32 ? resident_values(ar, r.src_a, v32_a, r.n_a, s) : resident_values(ar, r.src_a, v64_a, r.n_a, s);
+    if (f32) {
+        fill_slices(ar, r.t, r.n_t, r.n_blocks, r.piece, rp_t, ci_t, v32_t, s);
+        fill_slices(ar, r.a, r.n_a, r.n_blocks, r.piece, rp_a, ci_a, v32_a, s);
+    } else {
+        fill_slices(ar, r.t, r.n_t, r.n_blocks, r.piece, rp_t, ci_t, v64_t, s);
+        fill_slices(ar, r.a, r.n_a, r.n_blocks, r.piece, rp_a, ci_a, v64_a, s);
+    }
 }
 
 VecDev DeviceMatrix::make_vec(DeviceArena& ar, bool transpose, int lane_nnz, int64_t min_items) const {

@@ -176,18 +176,23 @@ class DeviceMatrix {
     // (build_vec_items), with zeroed piece slots and counters; items of four times the
     // default rows when min_items > 0 and that still gives at least min_items items.
     VecDev make_vec(DeviceArena& ar, bool transpose, int lane_nnz, int64_t min_items) const;
-    // The resident window's layout of both sides (deal_resident) for n_blocks blocks,
-    // without its values; false when a block's share of either side would need more than
-    // max_smem bytes of shared memory.
+    // A layout of both sides in slices on the device: the resident window's or a cluster's.
     struct Resident {
-        ResDev t, a;
-        const int32_t *src_t = nullptr, *src_a = nullptr;  // CSR position of each entry (-1: none)
-        int64_t n_t = 0, n_a = 0;                          // entries
+        ResDev t, a;  // indices and values once fill_resident() made them
+        int64_t n_t = 0, n_a = 0;  // entries
+        int32_t piece = 0;         // nonzeros per slice of a long row
         int n_blocks = 0;
         uint32_t smem = 0;  // dynamic shared memory of the largest block
     };
-    bool make_resident(DeviceArena& ar, int n_blocks, int esize, int ncv, int nrv, int par_bytes,
-                       uint32_t max_smem, Resident& out) const;
+    // The resident window's blocks, slices and rows of both sides (deal_resident) for
+    // n_blocks blocks, on the host; false when a block's share would need more than max_smem
+    // bytes of shared memory, else `smem` is what the largest needs.
+    bool plan_resident(int n_blocks, int esize, int ncv, int nrv, int par_bytes, uint32_t max_smem,
+                       HostResident& t, HostResident& a, uint32_t& smem) const;
+    // Upload such a plan, whose long rows are in pieces of `piece` nonzeros; the entries
+    // follow with fill_resident().
+    void upload_resident(DeviceArena& ar, const HostResident& t, const HostResident& a, int32_t piece,
+                         Resident& r) const;
     // The same for whole members in clusters (cluster_windows.cuh), each of as few blocks as
     // hold it, up to max_blocks: false when a member's blocks would need more than max_warps
     // slices or max_smem bytes of shared memory.  The members of one number of blocks form a
@@ -201,12 +206,9 @@ class DeviceMatrix {
     };
     bool make_cluster(DeviceArena& ar, int max_blocks, int esize, int max_warps, uint32_t max_smem, Resident& out,
                       std::vector<ClusterGroup>& groups) const;
-    // The entries' values from this matrix's values of the same precision.
+    // The entries, from this matrix's arrays on the device and its values of the same
+    // precision; stream-ordered.
     void fill_resident(DeviceArena& ar, Resident& r, bool f32, cudaStream_t s) const;
-  private:
-    void upload_resident(DeviceArena& ar, HostResident& t, HostResident& a, int lane_nnz, Resident& r) const;
-
-  public:
     // Build and upload A's long rows by column segment (build_seg) and a tiling of
     // their (segment, long row) pairs in stage geometry g, interleaved one block per
     // segment (interleave_tiles); false when no row qualifies.  `is_long` receives

@@ -265,7 +265,9 @@ struct HostResident {
 // them, or n_blocks of each instance in turn (per_member).  A row's lanes (about lane_nnz
 // nonzeros each), and with them the order in which its terms are added, depend on its
 // length alone, never on its block.  deal_resident makes the blocks, slices and rows
-// (which tell what a block's shared memory must hold), fill_resident then the entries.
+// (which tell what a block's shared memory must hold), fill_resident then the entries (the
+// device makes its own from the same slices, fill_slices_kernel; this form is its statement
+// on the host, which the layout's checks walk).
 // Slice depths are rounded up to a multiple of depth_unit.
 void deal_resident(const HostCsr& csr, const std::vector<int32_t>& inst_row_off, int n_blocks, int lane_nnz,
                    int depth_unit, bool per_member, HostResident& out);

@@ -808,7 +808,7 @@ ClusterForm& Projector::ensure_cluster() {
     return *f;
 }
 
-// The resident form of precision T, laid out the first time a window or a query asks.
+// The resident form of precision T, laid out the first time a window asks.
 template <typename T>
 ResidentForm& Projector::ensure_resident() {
     std::shared_ptr<ResidentForm>& f = std::is_same<T, float>::value ? res32_ : res64_;
@@ -819,7 +819,11 @@ ResidentForm& Projector::ensure_resident() {
 
 int32_t Projector::window_form() {
     if (tiny_ || vecwin_ || medium_ || !resident_) return tiny_ ? 3 : vecwin_ ? 2 : medium_ ? 1 : 0;
-    return (precision_ == PDFP_MIXED ? ensure_resident<float>() : ensure_resident<double>()).ready() ? 4 : 0;
+    auto fits = [&](auto prob, std::shared_ptr<ResidentForm>& f) {
+        if (!f) f = std::make_shared<ResidentForm>();
+        return f->plan<decltype(prob)>(M_, num_sms_, max_smem_block_);
+    };
+    return (precision_ == PDFP_MIXED ? fits(PdfpResident<float>{}, res32_) : fits(PdfpResident<double>{}, res64_)) ? 4 : 0;
 }
 
 template <>

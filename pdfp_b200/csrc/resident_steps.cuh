@@ -472,34 +472,45 @@ __global__ void __launch_bounds__(kResThreads, 1)
 
 // The resident form of one handle and precision on the host.
 struct ResidentForm {
-    bool tried = false;
-    DeviceMatrix::Resident r;  // n_blocks == 0: the handle does not fit
-    void* words = nullptr;     // the tagged x_bar (N) and z (M), and the give-up word
-    size_t words_bytes = 0;
+    DeviceMatrix::Resident r;  // n_blocks == 0: not laid out
     bool ready() const { return r.n_blocks > 0; }
 
-    // Lays the handle out for P's steps the first time, if it fits; stream-ordered.
+    // Whether the handle fits, decided the first time on the host: nothing goes to the device.
     template <class P>
-    void prepare(const DeviceMatrix& M, DeviceArena& ar, int num_sms, int max_smem_block, cudaStream_t stream) {
+    bool plan(const DeviceMatrix& M, int num_sms, int max_smem_block) {
         using T = typename P::T;
-        if (tried) return;
-        tried = true;
-        auto kern = resident_steps_kernel<P>;
-        int coop = 0, dev = 0, per_sm = 0;
-        PDFP_CK(cudaGetDevice(&dev));
-        PDFP_CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-        if (!coop || M.L.NNZ == 0) return;
+        if (planned_) return fits_;
+        planned_ = true;
+        if (M.L.NNZ == 0) return false;
         const uint32_t cap = static_cast<uint32_t>(max_smem_block) - 1024;  // its static memory
-        PDFP_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(cap)));
         // Where it stops to pay: 400 iterations of general-integer models, resident against
         // per-step launches, FP64 500k nonzeros (187 KB a block) 3.2 / 5.7 ms, 610k (about
         // 226 KB) 5.1 / 7.5; mixed 900k (194 KB) 4.5 / 6.3, 970k (200 KB) 4.6 / 6.4, 1M
         // (205 KB) 7.0 / 6.5: what shared memory takes, the gathers' misses lack in L1.
         const uint32_t most = sizeof(T) == 4 ? std::min(cap, 200u * 1024u) : cap;
+        if (!M.plan_resident(num_sms, sizeof(T), P::NCV, P::NRV, sizeof(ResPar<T>), most, t_, a_, smem_)) {
+            t_ = a_ = HostResident();
+            return false;
+        }
+        auto kern = resident_steps_kernel<P>;
+        int coop = 0, dev = 0, per_sm = 0;
+        PDFP_CK(cudaGetDevice(&dev));
+        PDFP_CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+        PDFP_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(cap)));
+        PDFP_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kResThreads, smem_));
+        fits_ = coop && per_sm >= 1;
+        return fits_;
+    }
+
+    // Lays the handle out for P's steps the first time, if it fits; stream-ordered.
+    template <class P>
+    void prepare(const DeviceMatrix& M, DeviceArena& ar, int num_sms, int max_smem_block, cudaStream_t stream) {
+        using T = typename P::T;
+        if (ready() || !plan<P>(M, num_sms, max_smem_block)) return;
         DeviceMatrix::Resident f;
-        if (!M.make_resident(ar, num_sms, sizeof(T), P::NCV, P::NRV, sizeof(ResPar<T>), most, f)) return;
-        PDFP_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kResThreads, f.smem));
-        if (per_sm < 1) return;
+        M.upload_resident(ar, t_, a_, 32 * kResLaneNnz, f);
+        t_ = a_ = HostResident();
+        f.smem = smem_;
         M.fill_resident(ar, f, std::is_same<T, float>::value, stream);
         words_bytes = sizeof(ResWord<T>) * (M.L.N + M.L.M) + 16;
         words = ar.alloc<unsigned char>(words_bytes);
@@ -531,6 +542,11 @@ struct ResidentForm {
     }
 
   private:
+    bool planned_ = false, fits_ = false;
+    HostResident t_, a_;  // from plan() to prepare()
+    uint32_t smem_ = 0;   // of the largest block
+    void* words = nullptr;     // the tagged x_bar (N) and z (M), and the give-up word
+    size_t words_bytes = 0;
     int64_t n_cols = 0, n_rows = 0;
 };
 

@@ -330,3 +330,49 @@ def test_members_of_several_sizes_in_clusters_of_their_own(oracle):
             s.solve(prm, 1.0)
         for name in ("pdhg_x", "pdhg_z", "current_y"):
             assert np.array_equal(s.get(name), both.get(p, name)), (p, name)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_the_first_solve_pays_for_the_layout(oracle, monkeypatch, precision):
+    """The first projection of a new handle, which lays the handle out for the resident window:
+    no slower than the same one in per-step launches (best of three handles each), although
+    it runs one window only."""
+    import time
+    milp, _, xt = synthetic.general_integer(1, m=24000, n=60000, m_eq=6000)
+    sc, is_eq, is_int, w = oracle.projector_inputs(milp)
+    probs = (sc.A, sc.con_ub, is_eq, is_int, sc.var_lb, sc.var_ub, w)
+    prm = SolverParameters(eps_optimal_relative=1e-9, eps_feasible_relative=1e-9, iteration_limit=200)
+    best = {}
+    for resident in ("0", "1") * 4:  # the first of each loads the kernels
+        s = _state(probs, precision, monkeypatch, resident)
+        s.set_target(xt / sc.D_c)
+        t = time.perf_counter()
+        s.solve(prm, 1.0)
+        best.setdefault(resident, []).append(time.perf_counter() - t)
+    assert min(best["1"][1:]) <= min(best["0"][1:])
+
+
+@pytest.mark.gpu
+def test_asking_for_the_window_form_leaves_the_device_alone():
+    """pdfp_get_window_form on a handle that has not solved: the answer is 4, and no device
+    memory goes to it (a process without the library's memory pool, which would hide it)."""
+    import sys
+    code = """
+import numpy as np, torch
+from pdfp_b200 import gpu, synthetic
+from oracle import oracle as O
+milp = synthetic.general_integer(1)[0]
+sc, is_eq, is_int, w = O.projector_inputs(milp)
+s = gpu.PDFPState(sc.A, sc.con_ub, is_eq, is_int, sc.var_lb, sc.var_ub, w)
+torch.cuda.synchronize()
+free = torch.cuda.mem_get_info()[0]
+form = gpu.C.c_int32()
+gpu.L.check(gpu.L.lib().pdfp_get_window_form(s._h, gpu.C.byref(form)))
+assert form.value == 4
+assert torch.cuda.mem_get_info()[0] == free
+"""
+    env = dict(os.environ, PDFP_POOL="0", PDFP_AUTOTUNE="0")
+    for name in ("PDFP_RESIDENT", "PDFP_STEP_ENGINE", "PDFP_TUNING"):
+        env.pop(name, None)
+    subprocess.run([sys.executable, "-c", code], check=True, cwd=ROOT, env=env)
