@@ -59,8 +59,11 @@ __device__ __forceinline__ void cluster_put(uint32_t a, int32_t v) {
     asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
 }
 // All threads of the cluster meet; what each wrote before (shared memory of any of its
-// blocks, global memory) is visible to all after.  The compiler's own barrier functions,
-// after a warp-wide join: every lane of a warp arrives at the same instruction.
+// blocks, global memory) is visible to all after.  A block of one member alone meets at its
+// barrier 0 by number: the warps of the columns, of the rows and idle ones arrive from
+// different places in the code, which __syncthreads() does not allow.  In a cluster the
+// compiler's barrier functions, after a warp-wide join: every lane of a warp arrives at the
+// same instruction.
 template <bool CL>
 __device__ __forceinline__ void cluster_meet() {
     if (CL) {
@@ -68,7 +71,7 @@ __device__ __forceinline__ void cluster_meet() {
         __cluster_barrier_arrive();
         __cluster_barrier_wait();
     } else {
-        __syncthreads();
+        asm volatile("barrier.sync 0;" ::: "memory");
     }
 }
 
