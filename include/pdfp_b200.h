@@ -295,7 +295,8 @@ PDFP_API int pdfp_get_tuning_seg(const pdfp_handle* h, int32_t* out);
  * from a captured graph; 1, one cooperative launch of the per-block row passes
  * (PDFP_MEDIUM=1); 2, one cooperative launch of the vec engine's warp items
  * (PDFP_VEC_WINDOW=1, both FP32 sides on the vec engine without long-row
- * pieces); 3, whole windows of each small member in one block's launch; 4, steps
+ * pieces); 3, whole windows of each small member in a thread-block cluster of
+ * one to eight blocks; 4, steps
  * 2 .. freq in one cooperative launch with the whole handle in the SMs' shared
  * memory (where it fits there and no switch names another form or engine;
  * PDFP_RESIDENT=0 switches it off). */
@@ -400,7 +401,8 @@ PDFP_API int pdfp_checker_destroy(pdfp_checker* c);
  * small kernel whose wait cannot complete -- which = 0: the tile engine's
  * mbarrier wait, on a phase that gets one arrival fewer than it expects;
  * which = 1: the cooperative window's grid barrier, expecting one block more
- * than launched -- with a limit of limit_seconds (0 < limit <= 4), no copy in
+ * than launched; which = 3: the resident window's wait for entries that nobody
+ * writes, whose threads must all have left it -- with a limit of limit_seconds (0 < limit <= 4), no copy in
  * flight.  Returns PDFP_E_TIMEOUT when the wait gave up as designed. */
 PDFP_API int pdfp_selftest_bounded_wait(int32_t which, double limit_seconds);
 

@@ -1778,7 +1778,7 @@ void Projector::solve(const pdfp_params* params, const double* primal_weights, p
         PDFP_CK(cudaStreamSynchronize(stream_));
         polled = true;
         dev_err = flags_h_[K_].status;
-        if (dev_err) throw Error(E_TIMEOUT, "a bounded device wait gave up (bulk copy did not complete)");
+        if (dev_err) throw Error(E_TIMEOUT, "a bounded device wait gave up (a copy, a barrier or an entry did not arrive)");
         if (timing_ && plan.run_b > plan.run_a && (with32 != with64)) {
             float run = 0.f, sp = 0.f, sd = 0.f;
             PDFP_CK(cudaEventElapsedTime(&run, tev_[0], tev_[1]));

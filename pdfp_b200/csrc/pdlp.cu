@@ -865,7 +865,7 @@ int32_t LpSolver::solve(double tolerance, double time_limit, int32_t sv_max_it, 
             PDFP_CK(cudaMemcpyAsync(fh, flags_, sizeof(InstFlags), cudaMemcpyDeviceToHost, stream_));
             PDFP_CK(cudaMemcpyAsync(&fh[1].status, err_, sizeof(int32_t), cudaMemcpyDeviceToHost, stream_));
             PDFP_CK(cudaStreamSynchronize(stream_));
-            if (fh[1].status) throw Error(E_TIMEOUT, "a bounded device wait gave up (bulk copy did not complete)");
+            if (fh[1].status) throw Error(E_TIMEOUT, "a bounded device wait gave up (a copy, a barrier or an entry did not arrive)");
             if (fh[0].status != ST_RUNNING) break;
             if (fh[0].polish_request && !polished_) {  // FP64 polish: convert and switch graphs
                 launch_elem(1, static_cast<int64_t>(n_) + m_, LpConvert<float, double>{v32_, v64_, n_, m_}, stream_);

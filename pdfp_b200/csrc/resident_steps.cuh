@@ -159,14 +159,30 @@ struct ResSide {
 };
 
 // After 64 fruitless looks: whether the wait is over for good.
-static __device__ __noinline__ bool res_gave_up(unsigned* dead, int32_t* err, uint64_t& t0) {
+static __device__ __noinline__ bool res_gave_up(unsigned* dead, int32_t* err, uint64_t& t0,
+                                                uint64_t limit_ns = kResWaitNs) {
     const uint64_t now = globaltimer_ns();
     if (t0 == 0) t0 = now;
     if (*reinterpret_cast<volatile unsigned*>(dead)) return true;
-    if (now - t0 <= kResWaitNs) return false;
+    if (now - t0 <= limit_ns) return false;
     atomicExch(dead, 1u);
     if (err) atomicExch(err, DEV_ERR_TIMEOUT);
     return true;
+}
+
+// Waits for an entry of step `want`; `off` once this or another wait gave up.
+template <typename T>
+__device__ __forceinline__ void res_wait(const ResWord<T>* entry, int32_t want, unsigned* dead, int32_t* err, bool& off,
+                                         uint64_t limit_ns = kResWaitNs) {
+    uint64_t t0 = 0;
+    unsigned spins = 0;
+    while (!off) {
+        T x;
+        int32_t t;
+        res_get(entry, x, t);
+        if (t == want) break;
+        if ((++spins & 63u) == 0) off = res_gave_up(dead, err, t0, limit_ns);
+    }
 }
 
 // A piece of a long row: the lanes' products pp[0], pp[32], .. (depth of them) and then the
@@ -281,15 +297,7 @@ __device__ __forceinline__ void res_pass(const P& prob, unsigned char* sm, const
     next_slice();
     if (lane == 0 && static_cast<int32_t>(threadIdx.x) < s.n_elem) {
         const int32_t c = idx[threadIdx.x];
-        uint64_t t0 = 0;
-        unsigned spins = 0;
-        while (c >= 0 && !off) {
-            T x;
-            int32_t t;
-            res_get(s.in + c, x, t);
-            if (t == want) break;
-            if ((++spins & 63u) == 0) off = res_gave_up(dead, prob.errp, t0);
-        }
+        if (c >= 0) res_wait(s.in + c, want, dead, prob.errp, off);
     }
     __syncwarp();
 #pragma unroll 1

@@ -72,7 +72,7 @@ def _out(out, size):
 
 def selftest_bounded_wait(which: int, limit_seconds: float = 0.05) -> int:
     """Run the library's bounded-wait self-test (pdfp_selftest_bounded_wait): 0 the
-    mbarrier wait, 1 the grid barrier.  Returns the status code (E_TIMEOUT when the
+    mbarrier wait, 1 the grid barrier, 3 the resident window's entries.  Returns the status code (E_TIMEOUT when the
     wait gave up as designed)."""
     return L.lib().pdfp_selftest_bounded_wait(int(which), float(limit_seconds))
 

@@ -51,3 +51,16 @@ def test_selftest_rejects_bad_arguments():
     assert gpu.selftest_bounded_wait(2, 0.05) == L.E_INVALID
     assert gpu.selftest_bounded_wait(0, 0.0) == L.E_INVALID
     assert gpu.selftest_bounded_wait(0, 5.0) == L.E_INVALID
+
+
+def test_the_resident_windows_wait_gives_up(oracle):
+    """Entries of a step that never comes: every thread of both blocks leaves its wait, those of
+    the block that did not reach the limit first by the abort word, and the GPU stays usable."""
+    before, xt = _handle(oracle, 1)
+    t = time.perf_counter()
+    assert gpu.selftest_bounded_wait(3, 0.05) == L.E_TIMEOUT
+    assert 0.05 <= time.perf_counter() - t < 3.0
+    assert b"bounded device wait gave up (self-test: entry)" in L.lib().pdfp_last_error()
+    p = SolverParameters(eps_optimal_relative=1e-4, eps_feasible_relative=1e-4)
+    before.set_target(xt)
+    assert before.solve(p, 1.0) == "OPTIMAL"
