@@ -118,3 +118,16 @@ def test_cupdlpx_rays_of_small_lps(oracle, case, m, n):
     assert so == ("PRIMAL_INFEASIBLE" if case == "infeasible" else "DUAL_INFEASIBLE")
     _, _, sg, ig = gpu.solve_lp_relaxation(milp, 1e-4, 30.0, True)
     assert (sg, ig) == (so, io)
+
+
+@pytest.mark.parametrize("tol", [1e-2, 1e-3])
+def test_cupdlpx_lp_that_fits_no_cluster(oracle, tol):
+    """A small LP with more slices (2,500 columns, 300 rows of 67 nonzeros) than a cluster has
+    warps, with the ray passes: one block runs its windows; the oracle's status, iterations
+    and objective."""
+    from pdfp_b200 import synthetic
+    milp, _, _ = synthetic.general_integer(2, m=300, n=2500, m_eq=75, mean_row=67.0)
+    _, _, so, io, ro = oracle.solve_lp_relaxation(milp, tol, 60.0, True)
+    _, _, sg, ig, rg = gpu.solve_lp_relaxation(milp, tol, 60.0, True, return_result=True)
+    assert (sg, ig) == (so, io)
+    assert rg["objective_value"] == pytest.approx(ro["objective_value"], rel=1e-8)

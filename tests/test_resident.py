@@ -376,3 +376,108 @@ assert torch.cuda.mem_get_info()[0] == free
     for name in ("PDFP_RESIDENT", "PDFP_STEP_ENGINE", "PDFP_TUNING"):
         env.pop(name, None)
     subprocess.run([sys.executable, "-c", code], check=True, cwd=ROOT, env=env)
+
+
+def _form(h):
+    from pdfp_b200 import gpu
+    form = gpu.C.c_int32()
+    gpu.L.check(gpu.L.lib().pdfp_get_window_form(h._h, gpu.C.byref(form)))
+    return form.value
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision,m", [("fp64", 24000), ("mixed", 36000)])
+def test_near_the_shared_memory_limit(oracle, monkeypatch, precision, m):
+    """Handles that fill their blocks' shared memory (600k nonzeros in FP64, 900k mixed), after
+    one and three windows: the bounds of the resident steps' test."""
+    milp, _, xt = synthetic.general_integer(3, m=m, n=5 * m // 2, m_eq=m // 4)
+    sc, is_eq, is_int, w = oracle.projector_inputs(milp)
+    probs = (sc.A, sc.con_ub, is_eq, is_int, sc.var_lb, sc.var_ub, w)
+    tol = 1e-10 if precision == "fp64" else 2e-4
+    s, o = _state(probs, precision, monkeypatch, "1"), oracle.OracleSolvers.PDFPState(*probs)
+    for windows in (1, 3):
+        prm = SolverParameters(eps_optimal_relative=1e-9, eps_feasible_relative=1e-9, iteration_limit=200 * windows)
+        for h in (s, o):
+            h.set_target(xt / sc.D_c)
+            h.solve(prm, 1.0)
+        assert s.total_count == 200 * windows
+        for name in ("pdhg_x", "pdhg_z", "current_y"):
+            a, b = s.get(name), o.get(name)
+            assert np.linalg.norm(a - b) <= tol * max(1.0, np.linalg.norm(b)), (windows, name)
+
+
+@pytest.mark.gpu
+def test_two_resident_handles_in_two_threads(oracle, monkeypatch):
+    """Two handles that each take the whole GPU, solved at the same time from two threads on
+    their own streams: the results of two others solved one after the other, bit for bit."""
+    import threading
+    monkeypatch.setenv("PDFP_AUTOTUNE", "0")
+    prm = SolverParameters(eps_optimal_relative=1e-9, eps_feasible_relative=1e-9, iteration_limit=1000)
+    inputs = []
+    for _, milp, xt in _models():
+        sc, is_eq, is_int, w = oracle.projector_inputs(milp)
+        inputs.append(((sc.A, sc.con_ub, is_eq, is_int, sc.var_lb, sc.var_ub, w), xt / sc.D_c))
+
+    def solve(s, xt, out):
+        for _ in range(3):  # each from the iterates of the one before
+            s.set_target(xt)
+            s.solve(prm, 1.0)
+            out.append([s.total_count] + [s.get(name) for name in ("pdhg_x", "current_y", "current_z")])
+
+    results = []
+    for together in (False, True):
+        work = [(_state(pr, "fp64", monkeypatch, "1"), xt, []) for pr, xt in inputs]
+        threads = [threading.Thread(target=solve, args=a) for a in work]
+        for t in threads:
+            t.start()
+            if not together:
+                t.join()
+        for t in threads:
+            t.join()
+        results.append([out for _, _, out in work])
+    for one, two in zip(*results):
+        assert len(one) == len(two) == 3
+        for a, b in zip(one, two):
+            assert a[0] == b[0] == 1000
+            for x, y in zip(a[1:], b[1:]):
+                assert np.array_equal(x, y)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_a_window_of_a_batch_member_equals_its_own_handles(oracle, monkeypatch, precision):
+    """One window, before any evaluation can change a step size: the members' iterates are their
+    single handles' bit for bit, with rows of one lane, of several and in pieces -- of the
+    members whose step size is their single handle's: the norm estimate's last bit is not
+    always the same in a batch, whose passes add partial sums of other tiles."""
+    from pdfp_b200 import gpu
+    monkeypatch.setenv("PDFP_RESIDENT", "1")
+    monkeypatch.setenv("PDFP_AUTOTUNE", "0")
+    monkeypatch.setenv("PDFP_MIXED_MIN_NNZ", "0")
+    models = synthetic.covering_packing_batch(seed=7, k=3, n_min=3000, n_max=9000)
+    models += [_models()[0][1], _models()[1][1]]
+    assert np.diff(models[-1].A.tocsr().indptr).max() > 1024
+    rng = np.random.default_rng(22)
+    prm = SolverParameters(eps_optimal_relative=1e-6, eps_feasible_relative=1e-6, iteration_limit=200)
+    probs, targets = [], []
+    for m in models:
+        sc, is_eq, is_int, w = oracle.projector_inputs(m)
+        probs.append((sc.A, sc.con_ub, is_eq, is_int, sc.var_lb, sc.var_ub, w))
+        targets.append(np.round(rng.random(len(m.c))) / sc.D_c)
+    b = gpu.PDFPBatch(probs, precision=precision)
+    assert _form(b) == 4
+    for p, xt in enumerate(targets):
+        b.set_target(p, xt)
+    b.solve(prm, 1.0)
+    compared = []
+    for p, pr in enumerate(probs):
+        s = gpu.PDFPState(*pr, precision=precision)
+        assert _form(s) == 4
+        s.set_target(targets[p])
+        s.solve(prm, 1.0)
+        if s.last["step_size"] != b.results[p]["step_size"]:
+            continue
+        compared.append(p)
+        for name in ("pdhg_x", "pdhg_y", "pdhg_z"):
+            assert np.array_equal(s.get(name), b.get(p, name)), (p, name)
+    assert len(compared) >= 3 and len(models) - 1 in compared  # the last one has the long rows
