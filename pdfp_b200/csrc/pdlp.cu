@@ -312,6 +312,7 @@ struct LpClusterRays : LpCluster<TT> {
 // or max_windows windows have run.  It reads the LP in global memory: one small enough for
 // a copy in shared memory fits a cluster.
 constexpr int kLpTinyWindowsPerLaunch = 64;
+constexpr int64_t kLpTinyMaxDim = 4096;  // rows + columns of a small LP
 
 template <typename T>
 __global__ void __launch_bounds__(kTinyThreads)
@@ -425,7 +426,7 @@ class LpSolver {
         M_.upload(ar_, f32_);  // unscaled; the FP32 copies are refreshed after the scaling
         {
             const char* te = std::getenv("PDFP_TINY");
-            tiny_ = !(te && te[0] == '0') && static_cast<int64_t>(A.m) + A.n <= 4096 &&
+            tiny_ = !(te && te[0] == '0') && static_cast<int64_t>(A.m) + A.n <= kLpTinyMaxDim &&
                     M_.L.NNZ <= (1 << 16);
             if (tiny_) {  // whole windows in a cluster, or else as a larger LP (cuPDLPx: one block)
                 if (f32_) prepare_cluster<float>(); else prepare_cluster<double>();
@@ -692,8 +693,9 @@ void LpSolver::launch_tiny_solve() {
     }
     const size_t smem = sizeof(double) * 2 * std::max(std::max(n_, m_), 1);
     auto kern = lp_tiny_solve_kernel<T>;
-    if (smem > 48 * 1024)
-        PDFP_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    // the same for every LP, so that another thread's LP never lowers it under this one
+    PDFP_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(sizeof(double) * 2 * kLpTinyMaxDim)));
     kern<<<1, kTinyThreads, smem, stream_>>>(*vp, d_, st_, flags_, M_.rp_t, M_.ci_t, M_.rp_a, M_.ci_a, n_,
                                              m_, err_, cupdlpx_ ? 1 : 0, kLpTinyWindowsPerLaunch);
     PDFP_CK(cudaGetLastError());
