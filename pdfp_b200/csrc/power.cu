@@ -195,8 +195,9 @@ std::vector<double> power_iteration(const DeviceMatrix& M, DeviceArena& ar,
     if (const char* te = std::getenv("PDFP_TINY")) tiny = tiny && te[0] != '0';
     if (tiny) {
         const size_t smem = sizeof(double) * static_cast<size_t>(smem_doubles);
+        // the same for every handle, so that another thread's never lowers it under this one
         PDFP_CK(cudaFuncSetAttribute(power_tiny_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(smem)));
+                                     static_cast<int>(sizeof(double) * 2 * kPowerTinyMaxDim)));
         power_tiny_kernel<<<K, kPowerTinyThreads, smem, stream>>>(b, M.rp_t, M.ci_t, M.v64_t, M.rp_a,
                                                                    M.ci_a, M.v64_a, M.row_off, M.col_off);
         PDFP_CK(cudaGetLastError());
