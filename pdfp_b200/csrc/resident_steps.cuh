@@ -25,8 +25,8 @@
 // (release, atomic, acquire, then the gathers) took 6.3 and 11 us.
 //
 // The order in which a row's terms are added depends on its length alone (its lanes
-// take every 2^lg-th term, then an xor tree; pieces of a long row in order), so a batch
-// member takes the steps of its own handle bit for bit.
+// take every 2^lg-th term, then an xor tree; pieces of a long row, which are summed in FP64,
+// in order), so a batch member with its own handle's step size takes its steps bit for bit.
 #pragma once
 #include <algorithm>
 #include <type_traits>
